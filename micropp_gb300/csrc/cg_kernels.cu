@@ -21,6 +21,9 @@
 namespace mgb {
 
 constexpr int kUpdRows = 4;  // rows per thread of the vector update
+// Largest batch (nodes of all its instances) solved by one cooperative launch: where the two forms' times per
+// iteration meet, at about 46^3 nodes (see k_cg_solve).
+constexpr long long kSolveNodes = 100000;
 
 __device__ __forceinline__ bool node_boundary(const MeshDev &m, int n, int &i, int &j, int &k) {
   i = n % m.nx;
@@ -197,6 +200,235 @@ __global__ void __launch_bounds__(kNodeBlock) k_cg_pupdate(MeshDev m, const Inst
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(active_count, 1u);
 }
 
+// ---------------------------------------------------------------------------------------------------
+// The whole solve in one cooperative launch, for batches whose iterations are shorter than three launches.
+//
+// A group of G blocks owns an instance and iterates on it alone: no lockstep with the other instances, no
+// launch between the phases.  The phases of an iteration (SpMV, vector update, p-update) are separated by a
+// barrier over the group's blocks; the cooperative launch keeps all blocks resident, and every wait is bounded.
+// Each block forms the scalars for itself from the partial sums, so a barrier is the only exchange.
+//
+// The FP64 pipe (2 lanes per SM and cycle: a warp instruction holds its quarter of the SM for 64 cycles) bounds
+// the work, so it is spread over as many SMs and schedulers as there are: a unit of the SpMV is 32 nodes x 3
+// rows on 3 warps, one row of 81 products per thread (one node per thread, as k_cg_spmv has it, leaves most SMs
+// idle on small grids and runs 243 products one after the other), and as few units per block as there are SMs for.  Every sum keeps the order of the launches of
+// one iteration (k_cg_spmv, k_cg_update, k_cg_pupdate): the products of a row, the lanes of a warp, the 8 warps
+// of a 256-thread block, the blocks -- so the solve is the same bit for bit.
+//
+// Microseconds per iteration of one instance, three launches against this kernel: 10^3 nodes 42 and 15, 20^3 47 and
+// 19, 30^3 59 and 37, 40^3 73 and 61, 50^3 102 and 101, 60^3 149 and 150 (there the FP64 pipe is full either way
+// and the launches need no barrier).  At 10^3 an iteration is 6 us of dependent FP64 products, 3.5 us of barriers
+// and 4 us of reduction trees, division and square root.
+
+constexpr int kUnitThreads = 96;   // 32 nodes x 3 rows
+constexpr unsigned int kSpinLimit = 1u << 22;
+
+__device__ __forceinline__ double ld_value(const double *p) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Barrier over the G blocks of a group: `ctr` counts arrivals, `target` the count that ends this barrier.  Returns
+// false (in every thread of the block) when the wait ran out.
+__device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int target, int *ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+    unsigned int spin = 0;
+    while ((int)(ld_acquire(ctr) - target) < 0 && ++spin < kSpinLimit) {
+    }
+    *ok = spin < kSpinLimit;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+// The sum over the blocks of a launch from its warp sums part[k * stride + w], as grid_finish<K> forms it; the
+// result is in sums[k * 8 + f] for the 8 warps f of the finishing block (sum8 adds them).
+template <int K>
+__device__ __forceinline__ void tree_blocks(const double *part, int stride, int nwarps, double (*sums)[8]) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, nblocks = (nwarps + 7) / 8;
+  for (int t = threadIdx.x >> 5; t < 8 * K; t += nw) {
+    const int f = t & 7, k = t >> 3;
+    double v = 0.0;
+    if (f * 32 < nblocks) {
+      for (int b = f * 32 + lane; b < nblocks; b += 256) {
+        double w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = (b * 8 + i < nwarps) ? __ldcg(part + (size_t)k * stride + b * 8 + i) : 0.0;
+        v += ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+    if (lane == 0) sums[k][f] = v;
+  }
+}
+
+__device__ __forceinline__ double sum8(const double *s, int nblocks) {
+  if (nblocks <= 32) return s[0];
+  return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+}
+
+// KMAX: units a block works on at a time, at most.
+template <int KMAX>
+__global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
+    k_cg_solve(MeshDev m, const Inst *insts, const int *list, int nlist, int G) {
+  __shared__ double sy[2][KMAX][2][32];
+  __shared__ double sums[2][8];
+  __shared__ double s_alpha, s_beta, s_rz;
+  __shared__ int s_its, s_done, s_ok;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int group = blockIdx.x / G, rank = blockIdx.x - group * G, ngroups = gridDim.x / G;
+  const int ug = wid / 3, fi = wid - ug * 3, K = nw / 3;
+  const int nrow = m.nn * 3, units = (m.nn + 31) / 32;
+  const int ublocks = (nrow + kUpdRows * kNodeBlock - 1) / (kUpdRows * kNodeBlock), ustride = ublocks * kNodeBlock;
+  const int uwarps = ublocks * (kNodeBlock / 32);
+  const size_t np = m.np;
+  for (int a = group; a < nlist; a += ngroups) {
+    const Inst &I = insts[list[a]];
+    CgState *cs = I.cg;
+    if (cs->done) continue;
+    double *part = I.red, *upart = I.red + units;
+    unsigned int *ctr = I.ticket, target = 0;
+    const double *vals = I.vals, *kinv = I.kinv;
+    double *x = I.du, *r = I.r, *z = I.z, *p = I.p, *Ap = I.Ap;
+    const double min_err = cs->min_err, rel_err = cs->rel_err, pnorm0 = cs->pnorm0;
+    const int max_its = cs->max_its;
+    if (threadIdx.x == 0) {
+      s_rz = cs->rz;
+      s_its = 0;
+    }
+    __syncthreads();
+    bool ok = true;
+    while (true) {
+      // Ap = A p and p.Ap
+      for (int u = rank * K + ug, turn = 0; u < units; u += G * K, turn ^= 1) {
+        const int n = u * 32 + lane;
+        double y = 0.0;
+        bool bn = true;
+        if (n < m.nn) {
+          int i, j, k;
+          bn = node_boundary(m, n, i, j, k);
+          if (bn) {
+            y = p[n * 3 + fi];
+          } else {
+            const double *v = vals + (size_t)(fi * 3) * np + n;
+#pragma unroll(KMAX > 4 ? 3 : 9)
+            for (int s = 0; s < 27; ++s) {
+              const int nb = n + (s / 9 - 1) * m.nxny + ((s / 3) % 3 - 1) * m.nx + (s % 3 - 1);
+              const double *vs = v + (size_t)(s * 9) * np;
+              y = fma(ld_value(vs), p[nb * 3 + 0], y);
+              y = fma(ld_value(vs + np), p[nb * 3 + 1], y);
+              y = fma(ld_value(vs + 2 * np), p[nb * 3 + 2], y);
+            }
+          }
+          Ap[n * 3 + fi] = y;
+        }
+        if (fi > 0) sy[turn][ug][fi - 1][lane] = y;
+        asm volatile("bar.sync %0, 96;" ::"r"(ug + 1) : "memory");  // the unit's 3 warps
+        if (fi == 0) {
+          double t = 0.0;
+          if (n < m.nn) {
+            const double y1 = sy[turn][ug][0][lane], y2 = sy[turn][ug][1][lane];
+            if (bn)
+              t = fma(y2, y2, fma(y1, y1, y * y));
+            else
+              t = p[n * 3 + 0] * y + p[n * 3 + 1] * y1 + p[n * 3 + 2] * y2;
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+          if (lane == 0) part[u] = t;
+        }
+      }
+      target += G;
+      if (!(ok = group_barrier(ctr, target, &s_ok))) break;
+      tree_blocks<1>(part, 0, units, sums);
+      __syncthreads();
+      if (threadIdx.x == 0) s_alpha = s_rz / sum8(sums[0], (units + 7) / 8);
+      __syncthreads();
+      // x += alpha p; r -= alpha Ap; z = kinv r; z.z and r.z
+      const double alpha = s_alpha;
+      for (int w = wid * G + rank; w < uwarps; w += G * nw) {
+        double pv[kUpdRows], av[kUpdRows], rr[kUpdRows], xv[kUpdRows], kv[kUpdRows];
+#pragma unroll
+        for (int q = 0; q < kUpdRows; ++q) {
+          const int row = w * 32 + lane + q * ustride;
+          if (row < nrow) {
+            pv[q] = p[row]; av[q] = Ap[row]; rr[q] = r[row]; xv[q] = x[row]; kv[q] = kinv[row];
+          }
+        }
+        double zz = 0.0, rz = 0.0;
+#pragma unroll
+        for (int q = 0; q < kUpdRows; ++q) {
+          const int row = w * 32 + lane + q * ustride;
+          if (row < nrow) {
+            x[row] = fma(alpha, pv[q], xv[q]);
+            const double rn = fma(-alpha, av[q], rr[q]);
+            const double zn = kv[q] * rn;
+            r[row] = rn;
+            z[row] = zn;
+            zz = fma(zn, zn, zz);
+            rz = fma(rn, zn, rz);
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          zz += __shfl_down_sync(0xffffffffu, zz, o);
+          rz += __shfl_down_sync(0xffffffffu, rz, o);
+        }
+        if (lane == 0) {
+          upart[w] = zz;
+          upart[uwarps + w] = rz;
+        }
+      }
+      target += G;
+      if (!(ok = group_barrier(ctr, target, &s_ok))) break;
+      tree_blocks<2>(upart, uwarps, uwarps, sums);
+      __syncthreads();
+      if (threadIdx.x == 32) s_beta = sum8(sums[1], ublocks) / s_rz;
+      if (threadIdx.x == 0) {
+        const double tot = sum8(sums[0], ublocks), pnorm = sqrt(tot);
+        const int its = s_its + 1;
+        const bool met = pnorm < min_err || pnorm < pnorm0 * rel_err, bad = !isfinite(tot) || !isfinite(sum8(sums[1], ublocks));
+        s_its = its;
+        s_done = !(its < max_its) || met || bad;
+        if (rank == 0 && s_done) {
+          cs->pnorm = pnorm;
+          cs->its = its;
+          cs->done = 1;
+          I.out->cg_its = its;
+          I.out->cg_maxed = !(its < max_its) && !met;
+          if (bad) I.out->nonfinite = 1;
+        }
+      }
+      __syncthreads();
+      if (s_done) break;
+      if (threadIdx.x == 0) s_rz = sum8(sums[1], ublocks);
+      const double beta = s_beta;
+      for (int row = rank * blockDim.x + threadIdx.x; row < nrow; row += G * blockDim.x) p[row] = fma(beta, p[row], z[row]);
+      target += G;
+      if (!(ok = group_barrier(ctr, target, &s_ok))) break;
+    }
+    if (threadIdx.x == 0) {
+      if (!ok) {  // a block of the group never arrived: reported to the host, which clears the counter
+        cs->done = 1;
+        I.out->stalled = 1;
+      } else if (atomicAdd(ctr, 1u) == target + G - 1) {
+        *ctr = 0u;  // the last block to leave; the others have left every barrier
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // Setup leaves out.cg_its = 0 for instances that stop before the first iteration.
 __global__ void k_cg_init_out(const Inst *insts, const int *list, int nlist) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,6 +475,36 @@ int mgb_launch_cg_pupdate(const MeshDev *m, const Inst *insts, const int *list, 
   k_cg_pupdate<<<dim3(cdiv((size_t)m->nn * 3, kNodeBlock), nlist), kNodeBlock, 0, s>>>(*m, insts, list,
                                                                                          active_count);
   return (int)cudaGetLastError();
+}
+
+// The iterations of the listed instances after mgb_launch_cg_setup, to the end, in one cooperative launch.  Returns
+// -1 without launching where the batch is too large for it to pay (see kSolveNodes) or the device cannot hold it.
+int mgb_launch_cg_solve(const MeshDev *m, const Inst *insts, const int *list, int nlist, cudaStream_t s) {
+  if (nlist <= 0) return 0;
+  if ((long long)m->nn * nlist > kSolveNodes) return -1;
+  int dev = 0, sms = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop || sms < 1) {
+    cudaGetLastError();
+    return -1;
+  }
+  const int units = (int)cdiv(m->nn, 32);
+  // as few units per block as fit on the SMs (one block each), then as many blocks per instance as there are
+  int K = 8;
+  while (K > 1 && (long long)nlist * cdiv(units, K / 2) <= sms) K /= 2;
+  const int groups = nlist < sms ? nlist : sms;
+  int G = sms / groups;
+  if (G > (int)cdiv(units, K)) G = (int)cdiv(units, K);
+  MeshDev mesh = *m;
+  void *args[] = {&mesh, &insts, &list, &nlist, &G};
+  const void *f = K > 4 ? (const void *)k_cg_solve<8> : (const void *)k_cg_solve<4>;
+  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(groups * G), dim3(kUnitThreads * K), args, 0, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return -1;
+  }
+  return (int)e;
 }
 
 }  // extern "C"

@@ -83,7 +83,7 @@ struct InstOut {
   int nonfinite;       // a reduction produced NaN/Inf
   int cg_maxed;        // the last CG solve stopped at max_its
   int cg6_its;         // iterations of the last 6-RHS CG solve
-  int pad;
+  int stalled;         // a one-launch solve waited in vain for one of its blocks
 };
 
 // Geometric multigrid hierarchy of one instance (mixed form).  Level 0 is the fine grid (the instance's vals32,

@@ -54,7 +54,9 @@ int run_dpcg(const MeshDev &m, Inst *d_inst, int *d_list, unsigned int *d_count,
   chk((cudaError_t)mgb_launch_cg_setup(&m, d_inst, d_list, 1, s), "cg setup");
   const int chunk = (m.nn > 200000) ? 8 : 32;
   unsigned int count = 0;
-  for (int done = 0; done <= max_its; done += chunk) {
+  const int one = mgb_launch_cg_solve(&m, d_inst, d_list, 1, s);
+  if (one > 0) chk((cudaError_t)one, "cg solve");
+  for (int done = 0; one < 0 && done <= max_its; done += chunk) {
     for (int it = 0; it < chunk; ++it) {
       if (it == chunk - 1) chk(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), s), "count reset");
       chk((cudaError_t)mgb_launch_cg_spmv(&m, d_inst, d_list, 1, s), "cg spmv");
@@ -68,6 +70,7 @@ int run_dpcg(const MeshDev &m, Inst *d_inst, int *d_list, unsigned int *d_count,
   InstOut o{};
   chk(cudaMemcpyAsync(&o, d_out, sizeof(o), cudaMemcpyDeviceToHost, s), "out");
   chk(cudaStreamSynchronize(s), "sync");
+  if (o.stalled) chk(cudaErrorLaunchTimeout, "cg solve");
   return o.cg_its;
 }
 

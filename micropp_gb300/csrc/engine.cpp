@@ -658,6 +658,14 @@ void Engine::download_out() {
   for (size_t s = 0; s < slots_.size(); ++s)
     check(cudaMemcpyAsync(&h_out_[s], slots_[s].out, sizeof(InstOut), cudaMemcpyDeviceToHost, stream_), "out");
   sync();
+  for (size_t s = 0; s < slots_.size(); ++s)
+    if (h_out_[s].stalled) {
+      for (Slot &w : slots_) {
+        cudaMemsetAsync(w.ticket, 0, sizeof(unsigned int), stream_);
+        cudaMemsetAsync(w.out, 0, sizeof(InstOut), stream_);
+      }
+      throw std::runtime_error("a linear solve stalled: a block of its launch never arrived");
+    }
 }
 
 double Engine::listed_cg_its(const std::vector<int> &slots) {
@@ -878,6 +886,14 @@ void Engine::cg_solve(const std::vector<int> &slots) {
   const double upd_bytes = nrow * 11.0 * 8;
   const int chunk = (mesh_.nn > 200000) ? 8 : 32;
   int done_its = 0;
+  if (!timing_on()) {  // the per-kernel timers need the iterations launched kernel by kernel
+    const int e = mgb_launch_cg_solve(&mesh_, d_insts_, d_list_, n, stream_);
+    if (e >= 0) {
+      check_launch(e, "cg solve");
+      launches_ += 1;
+      return;
+    }
+  }
   while (done_its <= cg_max_its_) {
     run_chunk(0, n, [&] {
       for (int it = 0; it < chunk; ++it) {

@@ -38,6 +38,11 @@ int mgb_launch_cg_update(const mgb::MeshDev *m, const mgb::Inst *insts, const in
 int mgb_launch_cg_pupdate(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist,
                           unsigned int *active_count, cudaStream_t s);
 
+// All iterations after mgb_launch_cg_setup in one cooperative launch, bit for bit those of the three launches
+// above; -1 (nothing launched) where that does not pay.  An instance whose out.stalled is set
+// afterwards was not solved, and its ticket is to be cleared.
+int mgb_launch_cg_solve(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
+
 int mgb_launch_assembly32(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
                           const float *ke_phase, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
 // FP32 Jacobian by node gather (every phase elastic or damage): k0g = wg B_g^T C B_g per phase and Gauss
