@@ -14,6 +14,7 @@
 
 #include "adjoint_laws.h"
 #include "bc.cuh"
+#include "coop.cuh"
 #include "device.cuh"
 #include "launch.h"
 #include "reduce.cuh"
@@ -382,6 +383,200 @@ __global__ void __launch_bounds__(kNodeBlock) k_bicg_r(MeshDev m, AdjDev A, unsi
   }
 }
 
+// The whole BiCGSTAB solve in one cooperative launch, for RVEs whose iterations are shorter than its 5 launches.
+//
+// The G blocks iterate together with a barrier between the phases (direction, K y, half step, K z, full step); each
+// block forms the scalars for itself from the blocks' partial sums.  A unit of 32 nodes is multiplied by 9 warps: one
+// of the 3 rows and one of the 3 planes of the stencil each, 27 products per thread -- the launched kernels' 243
+// products per thread keep a few SMs busy for tens of microseconds, since an FP64 warp instruction holds its quarter of
+// the SM for 64 cycles.  Rows 96 u .. 96 u + 95 of the vectors belong to the first 96 threads of unit u's group in
+// every phase.  A 12^3 J2 path of 4 steps, forward and reverse: 503 ms launched, 171 ms so.
+constexpr int kBicgUnit = 288;  // threads per unit
+constexpr int kBicgGroups = 3;  // units a block works on at a time, at most
+// Largest RVE (nodes) solved in one launch.
+constexpr int kBicgNodes = 100000;
+
+template <bool Transpose>
+__global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDev m, AdjDev A, int units) {
+  __shared__ double part_rows[2][kBicgGroups][9][32];
+  __shared__ double s_warp[2][kBicgUnit * kBicgGroups / 32];
+  __shared__ double s_tot[2], s_alpha, s_beta, s_omega, s_rho;
+  __shared__ int s_done, s_ok;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, G = gridDim.x, rank = blockIdx.x;
+  const int ug = tid / kBicgUnit, t = tid - ug * kBicgUnit, groups = blockDim.x / kBicgUnit, nwarps = blockDim.x >> 5;
+  const int fi = (t >> 5) % 3, dz = (t >> 5) / 3;
+  const int u0 = (int)((long long)units * rank / G), u1 = (int)((long long)units * (rank + 1) / G), nrow = 3 * m.nn;
+  const size_t np = m.np;
+  const double *vals = A.vals, *kinv = A.kinv, *rh = A.rh;
+  double *x = A.x, *r = A.r, *p = A.p, *v = A.v, *sv = A.s, *tv = A.t, *y = A.y, *z = A.z;
+  BicgState *st = A.st;
+  unsigned int *ctr = A.ticket, target = 0;
+  int its = 0, turn = 0, converged = st->converged;
+  const int max_its = st->max_its;
+  const double limit = st->rel_tol * st->r0;
+  double rnorm = st->rnorm;
+  bool ok = true;
+  if (tid == 0) {
+    s_rho = st->rho;
+    s_alpha = s_omega = 1.0;
+    s_beta = 0.0;
+    s_done = st->done;
+  }
+  __syncthreads();
+  const bool skip = s_done != 0;
+  auto barrier = [&]() {
+    target += G;
+    return ok = group_barrier(ctr, target, &s_ok);
+  };
+  // s_tot = the sums over all threads of a and b; partials in two buffers in turn, as a block may write the next ones
+  // while another still reads these.
+  auto reduce = [&](double a, double b) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+      s_warp[0][wid] = a;
+      s_warp[1][wid] = b;
+    }
+    __syncthreads();
+    double *part = A.red + (size_t)turn * 2 * G;
+    turn ^= 1;
+    if (tid < 2) {
+      double q = 0.0;
+      for (int w = 0; w < nwarps; ++w) q += s_warp[tid][w];
+      part[(size_t)tid * G + rank] = q;
+    }
+    if (!barrier()) return false;
+    if (wid < 2) {
+      double q = 0.0;
+      for (int b2 = lane; b2 < G; b2 += 32) q += __ldcg(part + (size_t)wid * G + b2);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) q += __shfl_down_sync(0xffffffffu, q, o);
+      if (lane == 0) s_tot[wid] = q;
+    }
+    __syncthreads();
+    return true;
+  };
+  // f(row) for the rows of this thread
+  auto each_row = [&](auto f) {
+    for (int u = u0 + ug; u < u1; u += groups)
+      if (t < 96 && u * 96 + t < nrow) f(u * 96 + t);
+  };
+  // f(row, (K in)_row) (K^T in) for the rows of this thread
+  auto product = [&](const double *in, auto f) {
+    int buf = 0;
+    for (int u = u0 + ug; u < u1; u += groups, buf ^= 1) {
+      const int n = u * 32 + lane;
+      int i, j, k;
+      double q = 0.0;
+      if (n < m.nn && !bnd(m, n, i, j, k)) {
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+          const int s = dz * 9 + e, nb = n + (dz - 1) * m.nxny + (e / 3 - 1) * m.nx + (e % 3 - 1);
+          const double *a =
+              Transpose ? vals + (size_t)((26 - s) * 9 + fi) * np + nb : vals + (size_t)(s * 9 + fi * 3) * np + n;
+          const size_t step = Transpose ? 3 * np : np;
+          q = fma(ld_value(a), in[nb * 3], q);
+          q = fma(ld_value(a + step), in[nb * 3 + 1], q);
+          q = fma(ld_value(a + 2 * step), in[nb * 3 + 2], q);
+        }
+      }
+      part_rows[buf][ug][t >> 5][lane] = q;
+      asm volatile("bar.sync %0, %1;" ::"r"(ug + 1), "n"(kBicgUnit) : "memory");
+      const int row = u * 96 + t;
+      if (t < 96 && row < nrow) {
+        const int l = t / 3, d = t - l * 3;
+        const double sum = (part_rows[buf][ug][d][l] + part_rows[buf][ug][3 + d][l]) + part_rows[buf][ug][6 + d][l];
+        f(row, bnd(m, u * 32 + l, i, j, k) ? in[row] : sum);
+      }
+    }
+  };
+  while (!skip) {
+    // p = r + beta (p - omega v); y = kinv p
+    {
+      const double beta = s_beta, omega = s_omega;
+      each_row([&](int row) {
+        const double q = r[row] + beta * (p[row] - omega * v[row]);
+        p[row] = q;
+        y[row] = kinv[row] * q;
+      });
+    }
+    if (!barrier()) break;
+    // v = K y; alpha = rho / (rh . v)
+    double a = 0.0, b = 0.0;
+    product(y, [&](int row, double q) {
+      v[row] = q;
+      a = fma(rh[row], q, a);
+    });
+    if (!reduce(a, 0.0)) break;
+    if (tid == 0) {
+      s_alpha = s_rho / s_tot[0];
+      if (!isfinite(s_alpha) || s_tot[0] == 0.0) s_done = 1;
+    }
+    __syncthreads();
+    if (s_done) break;
+    // x += alpha y; s = r - alpha v; z = kinv s
+    const double alpha = s_alpha;
+    each_row([&](int row) {
+      x[row] += alpha * y[row];
+      const double q = r[row] - alpha * v[row];
+      sv[row] = q;
+      z[row] = kinv[row] * q;
+    });
+    if (!barrier()) break;
+    // t = K z; omega = (t . s) / (t . t)
+    a = b = 0.0;
+    product(z, [&](int row, double q) {
+      tv[row] = q;
+      a = fma(q, sv[row], a);
+      b = fma(q, q, b);
+    });
+    if (!reduce(a, b)) break;
+    if (tid == 0) {
+      s_omega = s_tot[0] / s_tot[1];
+      if (!isfinite(s_omega) || s_tot[1] == 0.0) s_done = 1;
+    }
+    __syncthreads();
+    if (s_done) break;
+    // x += omega z; r = s - omega t; rho, beta and the stop test
+    const double omega = s_omega;
+    a = b = 0.0;
+    each_row([&](int row) {
+      x[row] += omega * z[row];
+      const double q = sv[row] - omega * tv[row];
+      r[row] = q;
+      a = fma(rh[row], q, a);
+      b = fma(q, q, b);
+    });
+    if (!reduce(a, b)) break;
+    its += 1;
+    rnorm = sqrt(s_tot[1]);
+    converged = rnorm <= limit;
+    if (tid == 0) {
+      const double rho = s_tot[0];
+      s_beta = (rho / s_rho) * (s_alpha / s_omega);
+      s_rho = rho;
+      s_done = converged || !(its < max_its) || !isfinite(s_tot[1]) || rho == 0.0;
+    }
+    __syncthreads();
+    if (s_done) break;
+  }
+  if (tid == 0 && !skip) {
+    if (rank == 0) {
+      st->its = its;
+      st->converged = converged;
+      st->rnorm = rnorm;
+      st->done = 1;
+    }
+    if (!ok)
+      st->stalled = 1;  // a block never arrived: reported to the host, which clears the counter
+    else if (atomicAdd(ctr, 1u) == target + G - 1)
+      *ctr = 0u;  // the last block to leave; the others have left every barrier
+  }
+}
+
 }  // namespace mgb
 
 using namespace mgb;
@@ -435,6 +630,25 @@ int mgb_launch_bicg_iter(const MeshDev *m, const AdjDev *A, unsigned int *active
     k_bicg_t<false><<<gn, kNodeBlock, 0, s>>>(*m, *A);
   k_bicg_r<<<gr, kNodeBlock, 0, s>>>(*m, *A, active);
   return (int)cudaGetLastError();
+}
+
+// All iterations after mgb_launch_bicg_init in one cooperative launch; -1 (nothing launched) where that does not pay.
+int mgb_launch_bicg_solve(const MeshDev *m, const AdjDev *A, int transpose, cudaStream_t s) {
+  const int sms = coop_sms();
+  if (!sms || m->nn > kBicgNodes) return -1;
+  int units = (int)cdiv(m->nn, 32);
+  const int per = (int)cdiv(units, sms), groups = per < kBicgGroups ? per : kBicgGroups;
+  const int blocks = (int)cdiv(units, groups) < sms ? (int)cdiv(units, groups) : sms;
+  MeshDev mesh = *m;
+  AdjDev adj = *A;
+  void *args[] = {&mesh, &adj, &units};
+  const void *f = transpose ? (const void *)k_bicg_solve<true> : (const void *)k_bicg_solve<false>;
+  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(kBicgUnit * groups), args, 0, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return -1;
+  }
+  return (int)e;
 }
 
 }  // extern "C"

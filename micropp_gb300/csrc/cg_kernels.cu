@@ -14,6 +14,7 @@
 // and their x values come through L1/L2.  Boundary rows are identity rows.
 #include <cuda_runtime.h>
 
+#include "coop.cuh"
 #include "device.cuh"
 #include "launch.h"
 #include "reduce.cuh"
@@ -211,9 +212,9 @@ __global__ void __launch_bounds__(kNodeBlock) k_cg_pupdate(MeshDev m, const Inst
 // The FP64 pipe (2 lanes per SM and cycle: a warp instruction holds its quarter of the SM for 64 cycles) bounds
 // the work, so it is spread over as many SMs and schedulers as there are: a unit of the SpMV is 32 nodes x 3
 // rows on 3 warps, one row of 81 products per thread (one node per thread, as k_cg_spmv has it, leaves most SMs
-// idle on small grids and runs 243 products one after the other), and as few units per block as there are SMs for.  Every sum keeps the order of the launches of
-// one iteration (k_cg_spmv, k_cg_update, k_cg_pupdate): the products of a row, the lanes of a warp, the 8 warps
-// of a 256-thread block, the blocks -- so the solve is the same bit for bit.
+// idle on small grids and runs 243 products one after the other), and as few units per block as there are SMs for.
+// Every sum keeps the order of the launches of one iteration (k_cg_spmv, k_cg_update, k_cg_pupdate): the products of a
+// row, the lanes of a warp, the 8 warps of a 256-thread block, the blocks -- so the solve is the same bit for bit.
 //
 // Microseconds per iteration of one instance, three launches against this kernel: 10^3 nodes 42 and 15, 20^3 47 and
 // 19, 30^3 59 and 37, 40^3 73 and 61, 50^3 102 and 101, 60^3 149 and 150 (there the FP64 pipe is full either way
@@ -221,34 +222,6 @@ __global__ void __launch_bounds__(kNodeBlock) k_cg_pupdate(MeshDev m, const Inst
 // and 4 us of reduction trees, division and square root.
 
 constexpr int kUnitThreads = 96;   // 32 nodes x 3 rows
-constexpr unsigned int kSpinLimit = 1u << 22;
-
-__device__ __forceinline__ double ld_value(const double *p) {
-  double v;
-  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
-__device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Barrier over the G blocks of a group: `ctr` counts arrivals, `target` the count that ends this barrier.  Returns
-// false (in every thread of the block) when the wait ran out.
-__device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int target, int *ok) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
-    unsigned int spin = 0;
-    while ((int)(ld_acquire(ctr) - target) < 0 && ++spin < kSpinLimit) {
-    }
-    *ok = spin < kSpinLimit;
-  }
-  __syncthreads();
-  return *ok != 0;
-}
 
 // The sum over the blocks of a launch from its warp sums part[k * stride + w], as grid_finish<K> forms it; the
 // result is in sums[k * 8 + f] for the 8 warps f of the finishing block (sum8 adds them).
@@ -482,13 +455,8 @@ int mgb_launch_cg_pupdate(const MeshDev *m, const Inst *insts, const int *list, 
 int mgb_launch_cg_solve(const MeshDev *m, const Inst *insts, const int *list, int nlist, cudaStream_t s) {
   if (nlist <= 0) return 0;
   if ((long long)m->nn * nlist > kSolveNodes) return -1;
-  int dev = 0, sms = 0, coop = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop || sms < 1) {
-    cudaGetLastError();
-    return -1;
-  }
+  const int sms = coop_sms();
+  if (!sms) return -1;
   const int units = (int)cdiv(m->nn, 32);
   // as few units per block as fit on the SMs (one block each), then as many blocks per instance as there are
   int K = 8;

@@ -139,6 +139,7 @@ struct Voigt6 {
 struct BicgState {
   double rho, rho_old, alpha, omega, beta, r0, rnorm, rel_tol;
   int its, max_its, done, converged;
+  int stalled, pad;     // a one-launch solve waited in vain for one of its blocks
 };
 
 // Vectors and scratch of the adjoint solve of one RVE (node-interleaved FP64, like u).

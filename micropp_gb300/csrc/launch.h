@@ -137,6 +137,9 @@ int mgb_launch_axpy(int n, double *x, const double *y, double a, cudaStream_t s)
 int mgb_launch_bicg_init(const mgb::MeshDev *m, const mgb::AdjDev *A, cudaStream_t s);
 int mgb_launch_bicg_iter(const mgb::MeshDev *m, const mgb::AdjDev *A, unsigned int *active, int transpose,
                          cudaStream_t s);
+// All iterations after mgb_launch_bicg_init in one cooperative launch; -1 (nothing launched) where that does not pay.
+// Where the state's `stalled` is set afterwards nothing was solved, and the ticket is to be cleared.
+int mgb_launch_bicg_solve(const mgb::MeshDev *m, const mgb::AdjDev *A, int transpose, cudaStream_t s);
 
 #ifdef __cplusplus
 }

@@ -211,7 +211,12 @@ int Engine::bicg_solve(bool transpose, double *x) {
   launches_ += 1;
   check_launch(mgb_launch_bicg_init(&mesh_, &P.adj, stream_), "bicg init");
   const int chunk = 16;
-  for (int done = 0; done <= kAdjMaxIts; done += chunk) {
+  const int one = mgb_launch_bicg_solve(&mesh_, &P.adj, transpose ? 1 : 0, stream_);
+  if (one >= 0) {
+    check_launch(one, "bicg solve");
+    launches_ += 1;
+  }
+  for (int done = 0; one < 0 && done <= kAdjMaxIts; done += chunk) {
     check(cudaMemsetAsync(d_count_, 0, sizeof(unsigned int), stream_), "count reset");
     for (int it = 0; it < chunk; ++it) {
       launches_ += 5;
@@ -224,6 +229,10 @@ int Engine::bicg_solve(bool transpose, double *x) {
   check(cudaMemcpyAsync(&st, P.d_st, sizeof(st), cudaMemcpyDeviceToHost, stream_), "bicg state");
   sync();
   P.adj.x = x_buf;
+  if (st.stalled) {
+    cudaMemsetAsync(w.ticket, 0, sizeof(unsigned int), stream_);
+    throw std::runtime_error("a linear solve stalled: a block of its launch never arrived");
+  }
   last_bicg_converged_ = st.converged != 0;
   return st.its;
 }
