@@ -526,10 +526,10 @@ void Engine::ensure_slots(int n) {
       if (gather32_) w.gpd = dalloc<float>((size_t)64 * mesh_.nelem, "Gauss-point tangent terms");
     }
     if (mixed) {
-      w.r32 = dalloc<float>(nd, "r32");
-      w.z32 = dalloc<float>(nd, "z32");
-      w.p32 = dalloc<float>(nd, "p32");
-      w.Ap32 = dalloc<float>(nd, "Ap32");
+      w.r32 = dalloc<float>((size_t)3 * mesh_.np, "r32");
+      w.z32 = dalloc<float>((size_t)3 * mesh_.np, "z32");
+      w.p32 = dalloc<float>((size_t)3 * mesh_.np, "p32");
+      w.Ap32 = dalloc<float>((size_t)3 * mesh_.np, "Ap32");
       w.du32 = dalloc<float>(nd, "du32");
     }
     if (implicit) {
@@ -575,6 +575,8 @@ void Engine::ensure_slots(int n) {
         h.lv[l].x = buf((size_t)18 * np, "multigrid vector");
         h.lv[l].y = buf((size_t)18 * np, "multigrid vector");
         h.lv[l].t = buf((size_t)18 * np, "multigrid vector");
+        for (float *v : {h.lv[l].b, h.lv[l].x, h.lv[l].y, h.lv[l].t})  // zero on boundary nodes from the start
+          check(cudaMemsetAsync(v, 0, (size_t)18 * np * sizeof(float), stream_), "multigrid vector");
       }
       w.mg = dalloc<MgInst>(1, "multigrid hierarchy");
       check(cudaMemcpy(w.mg, &h, sizeof(MgInst), cudaMemcpyHostToDevice), "multigrid hierarchy upload");
@@ -920,12 +922,36 @@ void Engine::cg_solve(const std::vector<int> &slots) {
   }
 }
 
+// Whether an FP32 solve of n listed instances runs in one cooperative launch: batches small enough, unless
+// per-kernel timers want the iterations launched kernel by kernel or the V-cycle reads the FP16 operator.
+bool Engine::coop32(int n, bool use_mg) const {
+  return !timing_on() && !(mg_ && use_mg && mg_half_) && mgb_coop_cg32_pays(&mesh_, n, mg_ && use_mg);
+}
+
+// That launch for the n instances in d_list_ (nr = 1: with the tolerances in d_eta_; nr = 6: after the tangent
+// residual kernel).  False when the device does not take it; nothing has run then.
+bool Engine::coop_solve32(int n, int nr, bool use_mg) {
+  const bool mg = mg_ && use_mg;
+  const int e = mgb_launch_coop_cg32(mg ? mg_mesh_.data() : &mesh_, mg ? (int)mg_mesh_.size() : 1, d_insts_, d_list_, n,
+                                     nr, d_eta_, cg_abs_tol_, mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_,
+                                     kMgCoarsePairs, stream_);
+  if (e < 0) return false;
+  check_launch(e, "cg solve (FP32)");
+  launches_ += 1;
+  return true;
+}
+
 // The mixed form's CG: FP32 values and vectors, FP64 dot products, same iteration and stop rule, with a
 // relative tolerance per slot.  use_mg: multigrid-preconditioned (when the handle has multigrid), capped at
 // kMgMaxIts iterations; otherwise Jacobi with cg_max_its.
 void Engine::cg_solve32(const std::vector<int> &slots, const std::vector<double> &rel_tols, bool use_mg) {
   const int n = (int)slots.size();
   const bool mg = mg_ && use_mg;
+  if (coop32(n, use_mg)) {
+    for (int a = 0; a < n; ++a) h_eta_[a] = rel_tols[a];
+    check(cudaMemcpyAsync(d_eta_, h_eta_, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "CG tolerances");
+    if (coop_solve32(n, 1, use_mg)) return;
+  }
   for (int a = 0; a < n; ++a) {
     CgState c{};
     c.min_err = cg_abs_tol_;
@@ -1180,10 +1206,11 @@ std::vector<int> Engine::tangent_solve(const std::vector<int> &slots, bool use_m
       timer_end(t_tan_);
     }
     const int nl = (int)live.size();
-    const int block = tuned_block(1, nl);
-    if (mg) mg_vcycle(6, nl, true, block);
+    const bool one_launch = coop32(nl, use_mg) && coop_solve32(nl, 6, use_mg);
+    const int block = one_launch ? 0 : tuned_block(1, nl);
+    if (mg && !one_launch) mg_vcycle(6, nl, true, block);
     int done_its = 0;
-    while (done_its <= cg_max_its_) {
+    while (!one_launch && done_its <= cg_max_its_) {
       run_chunk(mg ? 2 : 4, nl, [&] {
         for (int it = 0; it < chunk; ++it) {
           if (it == chunk - 1) check(cudaMemsetAsync(d_count_, 0, sizeof(unsigned int), stream_), "count reset");
@@ -1412,7 +1439,8 @@ std::vector<NewtonResult> Engine::newton(const std::vector<int> &slots,
     std::vector<int> mg_its(na, 0);  // iterations of multigrid solves redone with Jacobi
     // The mixed multigrid form runs the iteration's device work as one CUDA graph where it can (graphs on,
     // kernel timers off); otherwise kernel by kernel.
-    const bool fused = mixed && mg_ && graphs_ && !timing_on() && newton_graphs_ok_ && known_block(0, na) > 0;
+    const bool fused = mixed && mg_ && graphs_ && !timing_on() && newton_graphs_ok_ && known_block(0, na) > 0 &&
+                       !coop32(na, true);
     if (mixed) {
       if (!fused) assemble32(na);
     } else if (use_A0_ && !exact_tangent_ && res[idx[0]].its < its_with_A0_) {

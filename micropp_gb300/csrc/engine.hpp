@@ -171,6 +171,8 @@ class Engine {
   void download_out();
   void residual(const std::vector<int> &slots);
   void cg_solve(const std::vector<int> &slots);
+  bool coop32(int n, bool use_mg) const;
+  bool coop_solve32(int n, int nr, bool use_mg);
   void cg_solve32(const std::vector<int> &slots, const std::vector<double> &rel_tols, bool use_mg = true);
   std::vector<int> tangent_solve(const std::vector<int> &slots, bool use_mg = true);
   double slot_bytes() const;

@@ -77,6 +77,14 @@ int mgb_launch_t6_rhs(const mgb::MeshDev *m, const int *near, int nnear, const m
                       int nlist, cudaStream_t s);
 int mgb_launch_t6_residual(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, int x_zero,
                            int mg, cudaStream_t s);
+// All iterations of an FP32 CG solve of nr = 1 or 6 right-hand sides in one cooperative launch (coop_cg32.cu); levels:
+// the grids of the V-cycle, finest first (one level: Jacobi).  nr = 1: from b, with rel_tols[a] for the a-th listed
+// instance; nr = 6: from the state mgb_launch_t6_residual leaves.  An instance whose out.stalled is set afterwards
+// was not solved, and its ticket is to be cleared.  -1: not available, nothing launched.  _pays: whether it is the faster
+// form for a batch.
+int mgb_coop_cg32_pays(const mgb::MeshDev *m, int nlist, int mg);
+int mgb_launch_coop_cg32(const mgb::MeshDev *levels, int nlevels, const mgb::Inst *insts, const int *list, int nlist,
+                         int nr, const double *rel_tols, double abs_tol, int max_its, int pairs, cudaStream_t s);
 int mgb_launch_cg6_spmv(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, int block,
                         cudaStream_t s);
 int mgb_launch_cg6_update(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, int mg,
