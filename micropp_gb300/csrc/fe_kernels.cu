@@ -384,10 +384,11 @@ __global__ void __launch_bounds__(kNodeBlock) k_node_rhs(MeshDev m, const Inst *
 // and the order in which a matrix entry receives its (up to 8) contributions is fixed.  A block holds
 // kMatElems elements x 24 threads; thread p of an element owns row p of its Ke.
 //
-// Nonlinear laws: per Gauss point the tangent C (FD, 7 stress evaluations) is formed by 8 threads, then
-// cxb = (C B) wg is built cooperatively in shared memory and each thread accumulates its row
-// Ke[p][:] += B[:,p]^T cxb -- the reference's association (assembly.cpp:159-176).  Elastic-law elements
-// scatter the phase's precomputed Ke (identical for every element of a phase: B and wg are uniform).
+// Nonlinear laws: the tangents C of the block's 64 Gauss points are formed first, then cxb = (C B) wg is built
+// cooperatively in shared memory and each thread accumulates its row Ke[p][:] += B[:,p]^T cxb -- the reference's
+// association (assembly.cpp:159-176).  Elastic-law elements scatter the phase's precomputed Ke (identical for every
+// element of a phase: B and wg are uniform).  The FP64 pipe bounds the FP64 form: about 5,000 warp instructions per
+// block for the rows, 2,000 for the tangents.
 constexpr int kMatElems = 8;
 
 __device__ __forceinline__ int ell_idx(int s, int fi, int fj) { return s * 9 + fi * 3 + fj; }
@@ -415,6 +416,7 @@ __global__ void __launch_bounds__(kMatElems * 24) k_elem_mat(MeshDev m, Mats mat
   __shared__ double ue[kMatElems][24];
   __shared__ T Cg[kMatElems][8][36];
   __shared__ T cxb[kMatElems][6 * 24];
+  __shared__ int s_e[kMatElems], s_ph[kMatElems];  // element and phase; -1: no Gauss-point tangents to form
   for (int t = threadIdx.x; t < 192; t += blockDim.x) dsh[t] = dsh_g[t];
   const Inst &I = insts[list[blockIdx.y]];
   const int cx = color & 1, cy = (color >> 1) & 1, cz = (color >> 2) & 1;
@@ -436,32 +438,43 @@ __global__ void __launch_bounds__(kMatElems * 24) k_elem_mat(MeshDev m, Mats mat
     const int n = n0 + c_corner[a][2] * m.nxny + c_corner[a][1] * m.nx + c_corner[a][0];
     ue[el][p] = I.u[n * 3 + d];
   }
-  __syncthreads();
   const bool nonlin = valid && law != 0;
-  // Gauss-point tangents (FP64).
-  if (nonlin && p < 8) {
-    double eps[6], C[36];
-    gp_strain(&dsh[p * 24], ue[el], eps);
-    const double *vg = I.vars_old ? I.vars_old + ((size_t)e * 8 + p) * kNvarGp : nullptr;
-    if constexpr (Dual) {
-      const MatDev &md = mats.m[ph];
-      const double theta[adj::kNpar] = {md.E, md.nu, md.Xt, md.Sy, md.Ka};
-      double h[7], ds[6], dh[7];
+  if (p == 0) {
+    s_e[el] = nonlin ? e : -1;
+    s_ph[el] = ph;
+  }
+  __syncthreads();
+  // Gauss-point tangents (FP64): thread q of the block takes point q % 8 of element (q % 64) / 8, so that whole warps
+  // work, and the third q / 64 of its columns where a column is formed by itself (one stress evaluation or dual
+  // number each); the closed form is formed by the first 64 threads.
+  {
+    const int q = threadIdx.x & 63, third = threadIdx.x >> 6, tl = q >> 3, g = q & 7;
+    if (s_e[tl] >= 0 && (sizeof(T) == sizeof(double) || third == 0)) {
+      const MatDev &md = mats.m[s_ph[tl]];
+      double eps[6];
+      gp_strain(&dsh[g * 24], ue[tl], eps);
+      const double *vg = I.vars_old ? I.vars_old + ((size_t)s_e[tl] * 8 + g) * kNvarGp : nullptr;
+      T *C = Cg[tl][g];
+      if constexpr (Dual) {
+        const double theta[adj::kNpar] = {md.E, md.nu, md.Xt, md.Sy, md.Ka};
+        double h[7], ds[6], dh[7];
 #pragma unroll
-      for (int i = 0; i < 7; ++i) h[i] = vg ? vg[i] : 0.0;
+        for (int i = 0; i < 7; ++i) h[i] = vg ? vg[i] : 0.0;
 #pragma unroll 1
-      for (int j = 0; j < 6; ++j) {
-        adj::law_column(md.type, theta, eps, h, j, ds, dh);
+        for (int j = 2 * third; j < 2 * third + 2; ++j) {
+          adj::law_column(md.type, theta, eps, h, j, ds, dh);
 #pragma unroll
-        for (int i = 0; i < 6; ++i) C[i * 6 + j] = ds[i];
+          for (int i = 0; i < 6; ++i) C[i * 6 + j] = ds[i];
+        }
+      } else if constexpr (sizeof(T) == sizeof(float)) {
+        double Cd[36];
+        law_ctan_exact(md, eps, vg, Cd);  // mixed form: closed-form consistent tangent
+#pragma unroll
+        for (int i = 0; i < 36; ++i) C[i] = (T)Cd[i];
+      } else {
+        law_ctan_columns(md, eps, vg, 2 * third, C);  // FP64 form: the reference's forward differences
       }
-    } else if constexpr (sizeof(T) == sizeof(float)) {
-      law_ctan_exact(mats.m[ph], eps, vg, C);  // mixed form: closed-form consistent tangent
-    } else {
-      law_ctan(mats.m[ph], eps, vg, C);  // FP64 form: the reference's forward differences
     }
-#pragma unroll
-    for (int i = 0; i < 36; ++i) Cg[el][p][i] = (T)C[i];
   }
   __syncthreads();
   T row[24];

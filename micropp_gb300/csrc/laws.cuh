@@ -122,30 +122,17 @@ __device__ __forceinline__ void law_stress(const MatDev &m, const double *eps, c
   }
 }
 
-// get_ctan (material.cpp:84-95 closed form for the elastic law; forward differences of the stress with
-// step 1e-8 for J2 and damage, apply_perturbation material.cpp:48-63).  C is row-major 6x6.
-__device__ __forceinline__ void law_ctan(const MatDev &m, const double *eps, const double *vars, double *C) {
-  if (m.type == 0) {
-#pragma unroll
-    for (int i = 0; i < 36; ++i) C[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) C[i * 6 + j] = m.lambda;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) C[i * 6 + i] += m.two_mu;
-#pragma unroll
-    for (int i = 3; i < 6; ++i) C[i * 6 + i] = m.mu;
-    return;
-  }
+// Columns i0 and i0 + 1 of get_ctan for J2 and damage (material.cpp:84-95): forward differences of the stress with step
+// 1e-8 (apply_perturbation, material.cpp:48-63).  C is row-major 6x6.
+__device__ __forceinline__ void law_ctan_columns(const MatDev &m, const double *eps, const double *vars, int i0,
+                                                 double *C) {
   double s0[6];
   law_stress(m, eps, vars, s0);
 #pragma unroll 1
-  for (int i = 0; i < 6; ++i) {
+  for (int i = i0; i < i0 + 2; ++i) {
     double e1[6], s1[6];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) e1[j] = eps[j];
-    e1[i] += MGB_D_EPS_CTAN;
+    for (int j = 0; j < 6; ++j) e1[j] = (j == i) ? eps[j] + MGB_D_EPS_CTAN : eps[j];
     law_stress(m, e1, vars, s1);
 #pragma unroll
     for (int j = 0; j < 6; ++j) C[j * 6 + i] = (s1[j] - s0[j]) / MGB_D_EPS_CTAN;
