@@ -22,9 +22,12 @@
 namespace mgb {
 
 constexpr int kUpdRows = 4;  // rows per thread of the vector update
-// Largest batch (nodes of all its instances) solved by one cooperative launch: where the two forms' times per
-// iteration meet, at about 46^3 nodes (see k_cg_solve).
-constexpr long long kSolveNodes = 100000;
+// Largest batch (nodes of all its instances) solved by one cooperative launch: above, the two forms are equal (60^3 nodes)
+// or the launches faster (damage, plain form, 8 x 30^3 179 ms against 186, 32 x 20^3 191 against 210).
+constexpr long long kSolveNodes = 150000;
+// Microseconds of an iteration in one launch: a block's unit of 32 nodes (243 FP64 warp instructions of 64 cycles on
+// four quarters), the shortest unit (its chain of dependent products), and the rest.
+constexpr double kUnitUs = 2.0, kChainUs = 6.0, kPhasesUs = 9.0;
 
 __device__ __forceinline__ bool node_boundary(const MeshDev &m, int n, int &i, int &j, int &k) {
   i = n % m.nx;
@@ -216,10 +219,13 @@ __global__ void __launch_bounds__(kNodeBlock) k_cg_pupdate(MeshDev m, const Inst
 // Every sum keeps the order of the launches of one iteration (k_cg_spmv, k_cg_update, k_cg_pupdate): the products of a
 // row, the lanes of a warp, the 8 warps of a 256-thread block, the blocks -- so the solve is the same bit for bit.
 //
-// Microseconds per iteration of one instance, three launches against this kernel: 10^3 nodes 42 and 15, 20^3 47 and
-// 19, 30^3 59 and 37, 40^3 73 and 61, 50^3 102 and 101, 60^3 149 and 150 (there the FP64 pipe is full either way
-// and the launches need no barrier).  At 10^3 an iteration is 6 us of dependent FP64 products, 3.5 us of barriers
-// and 4 us of reduction trees, division and square root.
+// A block's units are a run, dealt over its groups of 3 warps.  p and z are component-major here (32 neighbours' entries
+// are two lines, not seven); the caller's buffers hold 3 np values for them.
+//
+// Microseconds per iteration of one instance, three launches against this kernel: 10^3 nodes 42 and 16, 30^3 57 and 30,
+// 40^3 72 and 56, 50^3 100 and 97, 60^3 149 and 145, 80^3 283 and 314 (there the FP64 pipe is full either way and the
+// launches need no barrier).  At 10^3 an iteration is 5 us of dependent FP64 products, 4 us of barriers and 5 us of
+// reduction trees, division and square root; at 50^3 73 us of products (54 at the pipe's measured rate).
 
 constexpr int kUnitThreads = 96;   // 32 nodes x 3 rows
 
@@ -232,11 +238,19 @@ __device__ __forceinline__ void tree_blocks(const double *part, int stride, int 
     const int f = t & 7, k = t >> 3;
     double v = 0.0;
     if (f * 32 < nblocks) {
-      for (int b = f * 32 + lane; b < nblocks; b += 256) {
-        double w[8];
+      for (int b = f * 32 + lane; b < nblocks; b += 512) {
+        double w[2][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) w[i] = (b * 8 + i < nwarps) ? __ldcg(part + (size_t)k * stride + b * 8 + i) : 0.0;
-        v += ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int e = (b + h * 256) * 8 + i;
+            w[h][i] = e < nwarps ? __ldcg(part + (size_t)k * stride + e) : 0.0;
+          }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (b + h * 256 < nblocks)
+            v += ((w[h][0] + w[h][4]) + (w[h][2] + w[h][6])) + ((w[h][1] + w[h][5]) + (w[h][3] + w[h][7]));
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -262,6 +276,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
   const int group = blockIdx.x / G, rank = blockIdx.x - group * G, ngroups = gridDim.x / G;
   const int ug = wid / 3, fi = wid - ug * 3, K = nw / 3;
   const int nrow = m.nn * 3, units = (m.nn + 31) / 32;
+  const int u0 = (int)((long long)units * rank / G), u1 = (int)((long long)units * (rank + 1) / G);
   const int ublocks = (nrow + kUpdRows * kNodeBlock - 1) / (kUpdRows * kNodeBlock), ustride = ublocks * kNodeBlock;
   const int uwarps = ublocks * (kNodeBlock / 32);
   const size_t np = m.np;
@@ -280,10 +295,14 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
       s_its = 0;
     }
     __syncthreads();
-    bool ok = true;
-    while (true) {
+    // p = z (as the setup left it), component-major from here on, as z from the first update
+    for (int u = u0 + ug; u < u1; u += K)
+      if (u * 32 + lane < m.nn) p[fi * np + u * 32 + lane] = z[(u * 32 + lane) * 3 + fi];
+    target += G;
+    bool ok = group_barrier(ctr, target, &s_ok);
+    while (ok) {
       // Ap = A p and p.Ap
-      for (int u = rank * K + ug, turn = 0; u < units; u += G * K, turn ^= 1) {
+      for (int u = u0 + ug, turn = 0; u < u1; u += K, turn ^= 1) {
         const int n = u * 32 + lane;
         double y = 0.0;
         bool bn = true;
@@ -291,16 +310,16 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
           int i, j, k;
           bn = node_boundary(m, n, i, j, k);
           if (bn) {
-            y = p[n * 3 + fi];
+            y = p[fi * np + n];
           } else {
             const double *v = vals + (size_t)(fi * 3) * np + n;
 #pragma unroll(KMAX > 4 ? 3 : 9)
             for (int s = 0; s < 27; ++s) {
               const int nb = n + (s / 9 - 1) * m.nxny + ((s / 3) % 3 - 1) * m.nx + (s % 3 - 1);
               const double *vs = v + (size_t)(s * 9) * np;
-              y = fma(ld_value(vs), p[nb * 3 + 0], y);
-              y = fma(ld_value(vs + np), p[nb * 3 + 1], y);
-              y = fma(ld_value(vs + 2 * np), p[nb * 3 + 2], y);
+              y = fma(ld_value(vs), p[nb], y);
+              y = fma(ld_value(vs + np), p[np + nb], y);
+              y = fma(ld_value(vs + 2 * np), p[2 * np + nb], y);
             }
           }
           Ap[n * 3 + fi] = y;
@@ -314,7 +333,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
             if (bn)
               t = fma(y2, y2, fma(y1, y1, y * y));
             else
-              t = p[n * 3 + 0] * y + p[n * 3 + 1] * y1 + p[n * 3 + 2] * y2;
+              t = p[n] * y + p[np + n] * y1 + p[2 * np + n] * y2;
           }
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
@@ -333,34 +352,33 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
         double pv[kUpdRows], av[kUpdRows], rr[kUpdRows], xv[kUpdRows], kv[kUpdRows];
 #pragma unroll
         for (int q = 0; q < kUpdRows; ++q) {
-          const int row = w * 32 + lane + q * ustride;
+          const int row = w * 32 + lane + q * ustride, n = row / 3;
           if (row < nrow) {
-            pv[q] = p[row]; av[q] = Ap[row]; rr[q] = r[row]; xv[q] = x[row]; kv[q] = kinv[row];
+            pv[q] = p[(row - n * 3) * np + n]; av[q] = Ap[row]; rr[q] = r[row]; xv[q] = x[row]; kv[q] = kinv[row];
           }
         }
         double zz = 0.0, rz = 0.0;
 #pragma unroll
         for (int q = 0; q < kUpdRows; ++q) {
-          const int row = w * 32 + lane + q * ustride;
+          const int row = w * 32 + lane + q * ustride, n = row / 3;
           if (row < nrow) {
             x[row] = fma(alpha, pv[q], xv[q]);
             const double rn = fma(-alpha, av[q], rr[q]);
             const double zn = kv[q] * rn;
             r[row] = rn;
-            z[row] = zn;
+            z[(row - n * 3) * np + n] = zn;
             zz = fma(zn, zn, zz);
             rz = fma(rn, zn, rz);
           }
         }
+        // both warp sums in one tree: lanes 0-15 add up zz, 16-31 rz (half the FP64 additions, in the same order)
+        const bool upper = lane >= 16;
+        const double give = __shfl_xor_sync(0xffffffffu, upper ? zz : rz, 16);
+        double both = upper ? give + rz : zz + give;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          zz += __shfl_down_sync(0xffffffffu, zz, o);
-          rz += __shfl_down_sync(0xffffffffu, rz, o);
-        }
-        if (lane == 0) {
-          upart[w] = zz;
-          upart[uwarps + w] = rz;
-        }
+        for (int o = 8; o > 0; o >>= 1) both += __shfl_down_sync(0xffffffffu, both, o, 16);
+        if (lane == 0) upart[w] = both;
+        if (lane == 16) upart[uwarps + w] = both;
       }
       target += G;
       if (!(ok = group_barrier(ctr, target, &s_ok))) break;
@@ -386,7 +404,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
       if (s_done) break;
       if (threadIdx.x == 0) s_rz = sum8(sums[1], ublocks);
       const double beta = s_beta;
-      for (int row = rank * blockDim.x + threadIdx.x; row < nrow; row += G * blockDim.x) p[row] = fma(beta, p[row], z[row]);
+      for (int q = rank * blockDim.x + threadIdx.x; q < 3 * m.np; q += G * blockDim.x) p[q] = fma(beta, p[q], z[q]);
       target += G;
       if (!(ok = group_barrier(ctr, target, &s_ok))) break;
     }
@@ -458,12 +476,21 @@ int mgb_launch_cg_solve(const MeshDev *m, const Inst *insts, const int *list, in
   const int sms = coop_sms();
   if (!sms) return -1;
   const int units = (int)cdiv(m->nn, 32);
-  // as few units per block as fit on the SMs (one block each), then as many blocks per instance as there are
-  int K = 8;
-  while (K > 1 && (long long)nlist * cdiv(units, K / 2) <= sms) K /= 2;
-  const int groups = nlist < sms ? nlist : sms;
-  int G = sms / groups;
-  if (G > (int)cdiv(units, K)) G = (int)cdiv(units, K);
+  // groups of blocks that each take one instance after the other: the number that the iterations' times ask for
+  // (kUnitUs per unit of a block, at least kChainUs, and kPhasesUs of barriers and scalars)
+  int groups = 1, G = sms;
+  double least = 0.0;
+  for (int g = 1; g <= nlist && g <= sms; ++g) {
+    const int blocks = sms / g < units ? sms / g : units;
+    const double work = kUnitUs * cdiv(units, blocks);
+    const double t = cdiv(nlist, g) * ((work > kChainUs ? work : kChainUs) + kPhasesUs);
+    if (g == 1 || t < least) {
+      least = t;
+      groups = g;
+      G = blocks;
+    }
+  }
+  const int K = cdiv(units, G) < 8 ? (int)cdiv(units, G) : 8;
   MeshDev mesh = *m;
   void *args[] = {&mesh, &insts, &list, &nlist, &G};
   const void *f = K > 4 ? (const void *)k_cg_solve<8> : (const void *)k_cg_solve<4>;

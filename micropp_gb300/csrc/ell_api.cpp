@@ -99,8 +99,8 @@ extern "C" int micropp3_ell_solve_cgpd(const int nodes[3], const double *vals, c
     I.b = const_cast<double *>(b);
     I.du = x;
     I.r = (double *)alloc(nd * sizeof(double));
-    I.z = (double *)alloc(nd * sizeof(double));
-    I.p = (double *)alloc(nd * sizeof(double));
+    I.z = (double *)alloc((size_t)3 * m.np * sizeof(double));
+    I.p = (double *)alloc((size_t)3 * m.np * sizeof(double));
     I.Ap = (double *)alloc(nd * sizeof(double));
     I.kinv = (double *)alloc(nd * sizeof(double));
     I.red = (double *)alloc((size_t)nblocks * kRedStride * sizeof(double));

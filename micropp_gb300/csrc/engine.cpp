@@ -514,8 +514,8 @@ void Engine::ensure_slots(int n) {
     w.out = dalloc<InstOut>(1, "out");
     if (fp64) {
       w.r = dalloc<double>(nd, "r");
-      w.z = dalloc<double>(nd, "z");
-      w.p = dalloc<double>(nd, "p");
+      w.z = dalloc<double>((size_t)3 * mesh_.np, "z");
+      w.p = dalloc<double>((size_t)3 * mesh_.np, "p");
       w.Ap = dalloc<double>(nd, "Ap");
       w.kinv = dalloc<double>(nd, "kinv");
       w.vals = dalloc<double>((size_t)kEllPerNode * mesh_.np, "ELL values");

@@ -33,8 +33,8 @@ void Engine::ensure_fp64_slot0() {
   Slot &w = slots_[0];
   const size_t nd = nndim();
   if (!w.r) w.r = dalloc<double>(nd, "r");
-  if (!w.z) w.z = dalloc<double>(nd, "z");
-  if (!w.p) w.p = dalloc<double>(nd, "p");
+  if (!w.z) w.z = dalloc<double>((size_t)3 * mesh_.np, "z");
+  if (!w.p) w.p = dalloc<double>((size_t)3 * mesh_.np, "p");
   if (!w.Ap) w.Ap = dalloc<double>(nd, "Ap");
   if (!w.kinv) w.kinv = dalloc<double>(nd, "kinv");
   if (!w.vals) w.vals = dalloc<double>((size_t)kEllPerNode * mesh_.np, "ELL values");
