@@ -53,6 +53,8 @@ constexpr int kMgCoarsePairs = 4;
 constexpr int kMgChunk = 4;
 constexpr int kMgMaxIts = 100;
 
+constexpr size_t kRingBytes = (size_t)64 << 20;
+
 // A structured grid of nx x ny x nz nodes (the multigrid levels and the separable product's intermediates).
 static MeshDev grid_of(int nx, int ny, int nz) {
   MeshDev g{};
@@ -111,8 +113,7 @@ Engine::Engine(const micropp3_config &cfg) {
   build_materials(cfg);
   build_phase_stiffness();
   // The FP32 Jacobian (mixed precision or implicit ctan) is assembled by node gather from the residual's
-  // Gauss-point tangent terms when every phase in use is elastic or damage; a J2 phase keeps the element
-  // colouring assembly.
+  // Gauss-point tangent terms when every phase in use is elastic or damage; with a J2 phase by element matrices.
   gather32_ = precision_ == MICROPP3_MIXED || ctan_mode_ == MICROPP3_CTAN_IMPLICIT;
   for (int e = 0; e < mesh_.nelem && gather32_; ++e) gather32_ = mats_.m[etype_[e]].type != 1;
   // Multigrid levels: every axis of n elements coarsens to ceil(n / 2) while each axis keeps at least 4
@@ -238,8 +239,10 @@ Engine::Engine(const micropp3_config &cfg) {
     I.vals = d_A0_;
     upload_insts();
     upload_list({0});
-    launches_ += 9;
-    check_launch(mgb_launch_assembly(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, 1, stream_), "A0");
+    launches_ += 2;
+    check_launch(mgb_launch_assembly(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, 1, d_ring_, ring_bytes_,
+                                     stream_),
+                 "A0");
     I.vals = slots_[0].vals;
     upload_insts();
   }
@@ -275,6 +278,7 @@ Engine::~Engine() {
   dfree(d_etype_);
   dfree(d_dsh_);
   dfree(d_ke_);
+  dfree(d_ring_);
   dfree(d_ke32_);
   dfree(d_k0g32_);
   dfree(d_dsh32_);
@@ -482,6 +486,8 @@ double Engine::slot_bytes() const {
     b += 4.0 * (kEllPerNode * np + nd + (gather32_ ? 64.0 * mesh_.nelem : 0.0));
   if (precision_ == MICROPP3_MIXED) b += 4.0 * 5.0 * nd;
   if (ctan_mode_ == MICROPP3_CTAN_IMPLICIT) b += (8.0 * 2.0 + 4.0 * 5.0) * 18.0 * np;
+  if (precision_ == MICROPP3_FP64 || !gather32_)
+    b += (precision_ == MICROPP3_FP64 ? 8.0 : 4.0) * 2.0 * 576.0 * mesh_.nex * mesh_.ney;
   if (mg_) {
     b += 4.0 * 21.0 * np;
     for (size_t l = 1; l < mg_mesh_.size(); ++l) b += 4.0 * (kEllPerNode + 3.0 + 4.0 * 18.0) * mg_mesh_[l].np;
@@ -489,6 +495,21 @@ double Engine::slot_bytes() const {
     b += 4.0 * kEllPerNode * (grid_of(c.nx, mesh_.ny, mesh_.nz).np + grid_of(c.nx, c.ny, mesh_.nz).np);
   }
   return b;
+}
+
+// The ring of element matrices that an assembly of n instances works through: two element layers at least, as many as
+// kRingBytes hold beyond that (half of the L2), no more than there are.
+void Engine::ensure_ring(int n, size_t value_bytes) {
+  const size_t layer = (size_t)n * 576 * mesh_.nex * mesh_.ney * value_bytes;
+  const size_t bytes = std::max(2 * layer, std::min((mesh_.nez + 1) * layer, kRingBytes));
+  if (bytes <= ring_bytes_) return;
+  clear_graphs();  // captured assemblies hold the old ring
+  sync();
+  dfree(d_ring_);
+  d_ring_ = nullptr;
+  ring_bytes_ = 0;
+  d_ring_ = dalloc<char>(bytes, "element matrices");
+  ring_bytes_ = bytes;
 }
 
 void Engine::ensure_slots(int n) {
@@ -500,6 +521,7 @@ void Engine::ensure_slots(int n) {
   const int nblocks = std::max((3 * mesh_.nn + kNodeBlock - 1) / kNodeBlock, (mesh_.nelem * 8 + 127) / 128) + 8;
   const bool fp64 = precision_ == MICROPP3_FP64, mixed = precision_ == MICROPP3_MIXED;
   const bool implicit = ctan_mode_ == MICROPP3_CTAN_IMPLICIT;
+  if (fp64 || ((mixed || implicit) && !gather32_)) ensure_ring(n, fp64 ? 8 : 4);
   slots_.resize(n);
   for (int s = old; s < n; ++s) {
     Slot &w = slots_[s];
@@ -1001,7 +1023,7 @@ void Engine::cg_solve32(const std::vector<int> &slots, const std::vector<double>
   }
 }
 
-// Algorithmic bytes: the values written once, plus u and the history read once per element (colouring) or
+// Algorithmic bytes: the values written once, plus u and the history read once per element (element matrices) or
 // the Gauss-point tangent terms (8 floats per Gauss point) read once (gather).
 void Engine::assemble32(int nlist) {
   if (gather32_) {
@@ -1012,8 +1034,9 @@ void Engine::assemble32(int nlist) {
                  "assembly (FP32 gather)");
   } else {
     timer_begin(t_asm_, (double)nlist * (4.0 * kEllPerNode * mesh_.np + 8.0 * nndim() + 8.0 * nvars()));
-    launches_ += 9;
-    check_launch(mgb_launch_assembly32(&mesh_, &mats_, d_etype_, d_dsh_, d_ke32_, d_insts_, d_list_, nlist, stream_),
+    launches_ += 2;
+    check_launch(mgb_launch_assembly32(&mesh_, &mats_, d_etype_, d_dsh_, d_ke32_, d_insts_, d_list_, nlist, d_ring_,
+                                       ring_bytes_, stream_),
                  "assembly (FP32)");
   }
   timer_end(t_asm_);
@@ -1451,12 +1474,14 @@ std::vector<NewtonResult> Engine::newton(const std::vector<int> &slots,
       a0_iteration = true;
     } else {
       timer_begin(t_asm_, (double)na * (8.0 * kEllPerNode * mesh_.np + 8.0 * nndim() + 8.0 * nvars()));
-      launches_ += 9;
+      launches_ += 2;
       if (exact_tangent_)  // load paths: the exact consistent tangent (quadratic Newton)
-        check_launch(mgb_launch_assembly_dual(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, na, stream_),
+        check_launch(mgb_launch_assembly_dual(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, na, d_ring_,
+                                              ring_bytes_, stream_),
                      "assembly");
       else
-        check_launch(mgb_launch_assembly(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, na, stream_),
+        check_launch(mgb_launch_assembly(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, na, d_ring_,
+                                         ring_bytes_, stream_),
                      "assembly");
       timer_end(t_asm_);
     }

@@ -171,6 +171,7 @@ class Engine {
   void download_out();
   void residual(const std::vector<int> &slots);
   void cg_solve(const std::vector<int> &slots);
+  void ensure_ring(int n, size_t value_bytes);
   bool coop32(int n, bool use_mg) const;
   bool coop_solve32(int n, int nr, bool use_mg);
   void cg_solve32(const std::vector<int> &slots, const std::vector<double> &rel_tols, bool use_mg = true);
@@ -267,6 +268,8 @@ class Engine {
   KernelTimer t_rap_;  // multigrid operators after an assembly: smoother diagonals and Galerkin products
   KernelTimer t_tan_;  // FP64 kernels of the implicit ctan: right-hand sides, refinement residuals, ctan sums
   KernelTimer t_mg1_, t_mg6_, t_mgc_;  // V-cycles: level-0 passes (1 and 6 RHS), coarse levels and transfers
+  char *d_ring_ = nullptr;  // element matrices of a few layers (ensure_ring)
+  size_t ring_bytes_ = 0;
   PathState path_;
   bool graphs_ = true;                         // CG chunks replayed from captured CUDA graphs
   std::map<long, cudaGraphExec_t> graph_cache_;  // (solver, listed instances) -> executable graph

@@ -1,5 +1,5 @@
 // fe_kernels.cu -- finite-element kernels of the homogenization path (sm_103a): the FP64 form's residual and
-// colour-ordered assembly, the mixed form's double-float residual and FP32 assemblies, the history update.
+// element assembly, the mixed form's double-float residual and FP32 assemblies, the history update.
 //
 // Every kernel runs over a batch: blockIdx.y indexes the list of active instances, blockIdx.x tiles the
 // nodes or elements of one RVE.  Summation orders follow the reference where a sum is local (Gauss points of
@@ -377,12 +377,17 @@ __global__ void __launch_bounds__(kNodeBlock) k_node_rhs(MeshDev m, const Inst *
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Jacobian assembly into ELL (assembly.cpp:105-178, ell-common.cpp:166-198).
+// Jacobian assembly into ELL (assembly.cpp:105-178, ell-common.cpp:166-198), in two kernels over a few element layers at
+// a time: the 24x24 matrices of the layers' elements go to a scratch ring (k_elem_ke), then the rows of the nodes whose
+// elements are complete are summed from it (k_ke_gather).  An entry receives its (up to 8) contributions in a fixed
+// order, by the parity of ex, then ey, then ez.  A block of k_elem_ke holds kMatElems elements x 24 threads; thread p
+// of an element owns row p of its Ke.
 //
-// Elements are processed in 8 colours (parity of ex, ey, ez) so that two elements of one launch never share
-// a node: each launch adds its elements' 24x24 blocks into the rows of their interior nodes without atomics,
-// and the order in which a matrix entry receives its (up to 8) contributions is fixed.  A block holds
-// kMatElems elements x 24 threads; thread p of an element owns row p of its Ke.
+// The ring keeps a layer per instance that the next chunk of layers still needs, and is small enough to stay in L2;
+// each chunk is two launches.  Adding the matrices straight into the rows takes 8 launches, one per parity class (else
+// two elements would add into a row at once), which leave small grids with a few blocks each, and scattered
+// read-modify-writes.  us per assembly, so and now: 8 x damage 12^3 1016 and 538, J2 20^3 698 and 512, damage 60^3 7091
+// and 6719 (the FP64 pipe), FP32 J2 50^3 2377 and 1442, exact J2 12^3 745 and 179.
 //
 // Nonlinear laws: the tangents C of the block's 64 Gauss points are formed first, then cxb = (C B) wg is built
 // cooperatively in shared memory and each thread accumulates its row Ke[p][:] += B[:,p]^T cxb -- the reference's
@@ -409,29 +414,26 @@ __device__ __forceinline__ float *ell_values<float>(const Inst &I) {
 // accumulated in FP32.  Dual = true (T = double): the exact derivative of the stress, column by column with
 // forward-mode dual numbers (adjoint_laws.h), for the adjoint of a load path (a missing history reads as 0).
 template <typename T, bool Dual = false>
-__global__ void __launch_bounds__(kMatElems * 24) k_elem_mat(MeshDev m, Mats mats, const int8_t *etype,
-                                                              const double *dsh_g, const T *ke_phase,
-                                                              const Inst *insts, const int *list, int color) {
+__global__ void __launch_bounds__(kMatElems * 24) k_elem_ke(MeshDev m, Mats mats, const int8_t *etype,
+                                                             const double *dsh_g, const T *ke_phase, const Inst *insts,
+                                                             const int *list, int z0, int z1, T *ring, int layers) {
   __shared__ double dsh[8 * 24];
   __shared__ double ue[kMatElems][24];
-  __shared__ T Cg[kMatElems][8][36];
-  __shared__ T cxb[kMatElems][6 * 24];
+  __shared__ T pool[kMatElems * (8 * 36 + 6 * 24)];
+  T(*Cg)[8][36] = reinterpret_cast<T(*)[8][36]>(pool);
+  T(*cxb)[6 * 24] = reinterpret_cast<T(*)[6 * 24]>(pool + kMatElems * 8 * 36);
+  __shared__ long long s_out[kMatElems];  // offset of the element's matrix in the ring, -1: no element
   __shared__ int s_e[kMatElems], s_ph[kMatElems];  // element and phase; -1: no Gauss-point tangents to form
   for (int t = threadIdx.x; t < 192; t += blockDim.x) dsh[t] = dsh_g[t];
   const Inst &I = insts[list[blockIdx.y]];
-  const int cx = color & 1, cy = (color >> 1) & 1, cz = (color >> 2) & 1;
-  const int ncx = (m.nex - cx + 1) / 2, ncy = (m.ney - cy + 1) / 2, ncz = (m.nez - cz + 1) / 2;
-  const int nce = ncx * ncy * ncz;
   const int el = threadIdx.x / 24, p = threadIdx.x % 24;
-  const int ce = blockIdx.x * kMatElems + el;
-  const bool valid = ce < nce;
-  int ex = 0, ey = 0, ez = 0, e = 0, n0 = 0, law = 0, ph = 0;
+  const int L = m.nex * m.ney, ce = z0 * L + blockIdx.x * kMatElems + el;
+  const bool valid = ce < z1 * L;
+  int e = 0, law = 0, ph = 0;
+  if (p == 0) s_out[el] = valid ? ((long long)blockIdx.y * layers + ce / L % layers) * 576 * L + ce % L : -1;
   if (valid) {
-    ex = 2 * (ce % ncx) + cx;
-    ey = 2 * ((ce / ncx) % ncy) + cy;
-    ez = 2 * (ce / (ncx * ncy)) + cz;
-    e = (ez * m.ney + ey) * m.nex + ex;
-    n0 = ez * m.nxny + ey * m.nx + ex;
+    e = ce;
+    const int ex = e % m.nex, ey = (e / m.nex) % m.ney, ez = e / L, n0 = ez * m.nxny + ey * m.nx + ex;
     ph = etype[e];
     law = mats.m[ph].type;
     const int a = p / 3, d = p % 3;
@@ -521,22 +523,48 @@ __global__ void __launch_bounds__(kMatElems * 24) k_elem_mat(MeshDev m, Mats mat
     }
     __syncthreads();
   }
-  if (!valid) return;
-  // Scatter row p = (local node a, dof d) into the ELL row of node(a), unless it is a boundary row.
-  const int ai = c_corner[a][0], aj = c_corner[a][1], ak = c_corner[a][2];
-  const int gi = ex + ai, gj = ey + aj, gk = ez + ak;
-  if (is_boundary(m, gi, gj, gk)) return;
-  const int node = n0 + ak * m.nxny + aj * m.nx + ai;
-  T *vals = ell_values<T>(I);
+  // the matrices to the ring, entry-major: 8 consecutive elements' values of an entry together, through shared memory
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const int s = (c_corner[b][2] - ak + 1) * 9 + (c_corner[b][1] - aj + 1) * 3 + (c_corner[b][0] - ai + 1);
+  for (int h = 0; h < 2; ++h) {
 #pragma unroll
-    for (int fj = 0; fj < 3; ++fj) {
-      T *dst = &vals[(size_t)ell_idx(s, d, fj) * m.np + node];
-      *dst += row[b * 3 + fj];
+    for (int q = 0; q < 12; ++q) pool[(p * 12 + q) * 9 + el] = row[h * 12 + q];
+    __syncthreads();
+    for (int t = threadIdx.x; t < 288 * kMatElems; t += kMatElems * 24) {
+      const int pq = t >> 3, l = t & 7, entry = pq / 12 * 24 + h * 12 + pq % 12;
+      if (s_out[l] >= 0) ring[s_out[l] + (long long)entry * L] = pool[pq * 9 + l];
+    }
+    __syncthreads();
+  }
+}
+
+// The ELL rows of the nodes [n0, n1) from the element matrices in the ring; thread (n, s) forms the block of node n at
+// stencil slot s.  Rows of boundary nodes and of the padding are zero.
+template <typename T>
+__global__ void __launch_bounds__(kElemBlock) k_ke_gather(MeshDev m, const Inst *insts, const int *list, int n0, int n1,
+                                                          const T *ring, int layers) {
+  const int n = n0 + blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.z;
+  if (n >= n1) return;
+  const int i = n % m.nx, j = (n / m.nx) % m.ny, k = n / m.nxny, L = m.nex * m.ney;
+  const int sx = s % 3 - 1, sy = (s / 3) % 3 - 1, sz = s / 9 - 1;
+  T acc[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) acc[q] = (T)0;
+  if (n < m.nn && !is_boundary(m, i, j, k)) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      // the element of parity class c around the node, in which the node is corner o and the neighbour corner o + s
+      const int ox = (i ^ c) & 1, oy = (j ^ (c >> 1)) & 1, oz = (k ^ (c >> 2)) & 1;
+      if (((ox + sx) | (oy + sy) | (oz + sz)) & ~1) continue;
+      const int a = local_of(ox, oy, oz), b = local_of(ox + sx, oy + sy, oz + sz);
+      const T *src = ring + (((size_t)blockIdx.y * layers + (k - oz) % layers) * 576 + a * 72 + b * 3) * L +
+                     (j - oy) * m.nex + i - ox;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) acc[q] += src[(size_t)(q / 3 * 24 + q % 3) * L];
     }
   }
+  T *vals = ell_values<T>(insts[list[blockIdx.y]]);
+#pragma unroll
+  for (int q = 0; q < 9; ++q) vals[(size_t)(s * 9 + q) * m.np + n] = acc[q];
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -550,7 +578,7 @@ __global__ void __launch_bounds__(kMatElems * 24) k_elem_mat(MeshDev m, Mats mat
 // with K0_g = wg B_g^T C_phase B_g precomputed per phase and Gauss point, and (a_g, c_g, s_g) written by the
 // residual kernel (k_elem_rhs_df) at the same displacement.  The 8 warps of a block (one element position each) add their
 // blocks into the block's 32 node rows (27 slots x 9) in shared memory in a fixed order; the rows are then
-// written once, coalesced.  No colouring, atomics or zeroing pass; boundary nodes get their real rows.
+// written once, coalesced.  No element matrices, atomics or zeroing pass; boundary nodes get their real rows.
 constexpr int kAsmNodes = 32;
 constexpr int kAsmRow = kEllPerNode + 2;  // 245 floats: odd stride, conflict-free
 
@@ -705,14 +733,6 @@ __global__ void __launch_bounds__(kAsmNodes * 8) k_asm_gather32(MeshDev m, Mats 
   }
 }
 
-// Zero the ELL values of the listed instances (ell_set_zero_mat, ell-common.cpp:200).
-template <typename T>
-__global__ void k_zero_vals(size_t count, const Inst *insts, const int *list) {
-  T *v = ell_values<T>(insts[list[blockIdx.y]]);
-  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x)
-    v[t] = (T)0;
-}
-
 // ---------------------------------------------------------------------------------------------------
 // Internal-variable update (update.cpp:32-56), one thread per Gauss point; the nonlinear flags are OR-ed
 // into out.nonlinear.
@@ -796,17 +816,20 @@ using namespace mgb;
 static inline unsigned cdiv(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
 template <typename T, bool Dual = false>
-static int launch_assembly(const MeshDev *m, const Mats *mats, const int8_t *etype, const double *dsh, const T *ke_phase,
-                           const Inst *insts, const int *list, int nlist, cudaStream_t s) {
+static int launch_assembly(const MeshDev *m, const Mats *mats, const int8_t *etype, const double *dsh,
+                           const T *ke_phase, const Inst *insts, const int *list, int nlist, void *ring, size_t bytes,
+                           cudaStream_t s) {
   if (nlist <= 0) return 0;
-  const size_t count = (size_t)kEllPerNode * m->np;
-  k_zero_vals<T><<<dim3(cdiv(count, 8 * kNodeBlock), nlist), kNodeBlock, 0, s>>>(count, insts, list);
-  for (int c = 0; c < 8; ++c) {
-    const int cx = c & 1, cy = (c >> 1) & 1, cz = (c >> 2) & 1;
-    const int nce = ((m->nex - cx + 1) / 2) * ((m->ney - cy + 1) / 2) * ((m->nez - cz + 1) / 2);
-    if (nce <= 0) continue;
-    k_elem_mat<T, Dual><<<dim3(cdiv(nce, kMatElems), nlist), kMatElems * 24, 0, s>>>(*m, *mats, etype, dsh, ke_phase,
-                                                                                     insts, list, c);
+  const size_t L = (size_t)m->nex * m->ney, fit = bytes / (sizeof(T) * 576 * L * nlist);
+  const int layers = fit < (size_t)m->nez + 1 ? (int)fit : m->nez + 1;
+  if (!ring || layers < 2) return (int)cudaErrorInvalidValue;
+  for (int z0 = 0; z0 < m->nez; z0 += layers - 1) {
+    const int z1 = z0 + layers - 1 < m->nez ? z0 + layers - 1 : m->nez;
+    const int n0 = z0 * m->nxny, n1 = z1 < m->nez ? z1 * m->nxny : m->np;
+    k_elem_ke<T, Dual><<<dim3(cdiv((z1 - z0) * L, kMatElems), nlist), kMatElems * 24, 0, s>>>(
+        *m, *mats, etype, dsh, ke_phase, insts, list, z0, z1, (T *)ring, layers);
+    k_ke_gather<T><<<dim3(cdiv(n1 - n0, kElemBlock), nlist, 27), kElemBlock, 0, s>>>(*m, insts, list, n0, n1,
+                                                                                     (const T *)ring, layers);
   }
   return (int)cudaGetLastError();
 }
@@ -853,18 +876,21 @@ int mgb_launch_node_gather(const MeshDev *m, const Inst *insts, const int *list,
 }
 
 int mgb_launch_assembly(const MeshDev *m, const Mats *mats, const int8_t *etype, const double *dsh,
-                        const double *ke_phase, const Inst *insts, const int *list, int nlist, cudaStream_t s) {
-  return launch_assembly<double>(m, mats, etype, dsh, ke_phase, insts, list, nlist, s);
+                        const double *ke_phase, const Inst *insts, const int *list, int nlist, void *ring, size_t bytes,
+                        cudaStream_t s) {
+  return launch_assembly<double>(m, mats, etype, dsh, ke_phase, insts, list, nlist, ring, bytes, s);
 }
 
 int mgb_launch_assembly_dual(const MeshDev *m, const Mats *mats, const int8_t *etype, const double *dsh,
-                             const double *ke_phase, const Inst *insts, const int *list, int nlist, cudaStream_t s) {
-  return launch_assembly<double, true>(m, mats, etype, dsh, ke_phase, insts, list, nlist, s);
+                             const double *ke_phase, const Inst *insts, const int *list, int nlist, void *ring, size_t bytes,
+                        cudaStream_t s) {
+  return launch_assembly<double, true>(m, mats, etype, dsh, ke_phase, insts, list, nlist, ring, bytes, s);
 }
 
 int mgb_launch_assembly32(const MeshDev *m, const Mats *mats, const int8_t *etype, const double *dsh,
-                          const float *ke_phase, const Inst *insts, const int *list, int nlist, cudaStream_t s) {
-  return launch_assembly<float>(m, mats, etype, dsh, ke_phase, insts, list, nlist, s);
+                          const float *ke_phase, const Inst *insts, const int *list, int nlist, void *ring, size_t bytes,
+                        cudaStream_t s) {
+  return launch_assembly<float>(m, mats, etype, dsh, ke_phase, insts, list, nlist, ring, bytes, s);
 }
 
 int mgb_launch_assembly_gather32(const MeshDev *m, const Mats *mats, const int8_t *etype, const float *k0g,

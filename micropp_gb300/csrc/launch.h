@@ -23,11 +23,14 @@ int mgb_launch_copy(int n, const double *const *src, double *const *dst, const i
 // (the mixed form with elastic and damage phases only).
 int mgb_launch_residual(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
                         const mgb::Inst *insts, const int *list, int nlist, int form, cudaStream_t s);
+// ring: scratch of `bytes` for the element matrices, of two element layers of all instances at least.
 int mgb_launch_assembly(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
-                        const double *ke_phase, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
+                        const double *ke_phase, const mgb::Inst *insts, const int *list, int nlist, void *ring,
+                        size_t bytes, cudaStream_t s);
 // FP64 Jacobian with the exact Gauss-point tangents (forward-mode dual numbers), for the adjoint.
 int mgb_launch_assembly_dual(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
-                             const double *ke_phase, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
+                             const double *ke_phase, const mgb::Inst *insts, const int *list, int nlist, void *ring,
+                             size_t bytes, cudaStream_t s);
 int mgb_launch_evolve(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
                       const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
 int mgb_launch_elem_fields(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
@@ -44,7 +47,8 @@ int mgb_launch_cg_pupdate(const mgb::MeshDev *m, const mgb::Inst *insts, const i
 int mgb_launch_cg_solve(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
 
 int mgb_launch_assembly32(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
-                          const float *ke_phase, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
+                          const float *ke_phase, const mgb::Inst *insts, const int *list, int nlist, void *ring,
+                          size_t bytes, cudaStream_t s);
 // FP32 Jacobian by node gather (every phase elastic or damage): k0g = wg B_g^T C B_g per phase and Gauss
 // point [3][8][576], kesum = its sum over g per phase [3][576], dsh32 = the shape-function gradients [8][24].
 // sdiag = 1: also the multigrid's level-0 smoother diagonal, as mgb_launch_mg_sdiag(l = 0, omega, csafe).

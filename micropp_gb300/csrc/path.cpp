@@ -30,6 +30,7 @@ constexpr int kAdjMaxIts = 20000;
 // Slot 0 with the FP64 buffers of the plain form (a mixed-precision handle does not allocate them).
 void Engine::ensure_fp64_slot0() {
   ensure_slots(1);
+  ensure_ring(1, sizeof(double));
   Slot &w = slots_[0];
   const size_t nd = nndim();
   if (!w.r) w.r = dalloc<double>(nd, "r");
@@ -281,8 +282,9 @@ int Engine::path_vjp(const double *gsigma, double *grad_params, double *grad_str
       I.has_vars_old = 1;
       upload_insts();
       upload_list({0});
-      launches_ += 9;
-      check_launch(mgb_launch_assembly_dual(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, 1, stream_),
+      launches_ += 2;
+      check_launch(mgb_launch_assembly_dual(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, 1, d_ring_,
+                                            ring_bytes_, stream_),
                    "adjoint tangent");
       AdjStep st{};
       std::memcpy(st.g, gsigma + (size_t)n * 6, sizeof(st.g));
