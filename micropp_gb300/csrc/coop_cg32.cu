@@ -79,6 +79,7 @@ struct Ctx {
   const double *b;
   double *red;
   unsigned int *ctr;
+  uint64_t policy;  // L2 eviction priority of the matrix values
   double min_err, rel_err;
   double warp[2][kWarps], tot[12], rz[6], pn0[6];
   float alpha[6], beta[6];
@@ -170,13 +171,20 @@ __device__ __forceinline__ void row_products(int nx, int nxny, size_t np, V valu
   }
 }
 
-// The matrix values of unit u to shared memory, by `threads` threads of which this is the t-th; finished by the
-// caller's cp_wait and barrier.
-__device__ __forceinline__ void copy_unit(float *dst, const float *vals, size_t np, int u, int t, int threads) {
-  for (int q = t; q < kEllPerNode * 8; q += threads) {
-    const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst + q * 4);
-    const float *src = vals + (size_t)(q >> 3) * np + u * 32 + (q & 7) * 4;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+// The matrix values of unit u to shared memory, by the 96 threads of a group of which this is the t-th; finished by the
+// caller's cp_wait and barrier.  policy: the L2 eviction priority (see keep_fraction), 0 for the usual one.
+__device__ __forceinline__ void copy_unit(float *dst, const float *vals, size_t np, int u, int t, uint64_t policy) {
+  constexpr int kStep = 32 * kSubs / 8;  // rows per round of the group's threads, 8 of them to a row
+  unsigned int d = (unsigned int)__cvta_generic_to_shared(dst + t * 4);
+  const float *src = vals + (size_t)(t >> 3) * np + u * 32 + (t & 7) * 4;
+  const size_t step = kStep * np;
+  if (policy) {
+    for (int row = t >> 3; row < kEllPerNode; row += kStep, d += kStep * 128, src += step)
+      asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "l"(policy)
+                   : "memory");
+  } else {
+    for (int row = t >> 3; row < kEllPerNode; row += kStep, d += kStep * 128, src += step)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
   }
 }
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
@@ -258,7 +266,7 @@ __device__ __noinline__ void apply(int op, int l, int in_sel, int out_sel) {
     const int u = first + k * step, n = u * 32 + lane, want = l << 24 | u;
     if (c.held[group] != want) {
       asm volatile("bar.sync %0, 96;" ::"r"(group + 1) : "memory");
-      copy_unit(buf, A, np, u, sub * 32 + lane, 96);
+      copy_unit(buf, A, np, u, sub * 32 + lane, c.policy);
       if (sub == 0 && lane == 0) c.held[group] = want;
       cp_wait();
       asm volatile("bar.sync %0, 96;" ::"r"(group + 1) : "memory");
@@ -693,7 +701,7 @@ __device__ __noinline__ double2 setup1() {
 template <int NR, bool MG>
 __global__ void __launch_bounds__(kThreads, 1)
     k_coop_cg32(Levels lv, const Inst *insts, const int *list, int G, const double *rel_tols, double abs_tol,
-                int max_its_arg, int pairs) {
+                int max_its_arg, int pairs, float keep) {
   Ctx &c = ctx();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int a = blockIdx.x / G, rank = blockIdx.x - a * G;
@@ -704,6 +712,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     c.G = G;
     c.rank = rank;
     c.pairs = pairs;
+    uint64_t policy = 0;
+    if (keep < 1.f)
+      asm volatile("createpolicy.fractional.L2::evict_normal.L2::evict_first.b64 %0, %1;" : "=l"(policy) : "f"(keep));
+    c.policy = policy;
     c.workers = tail ? G - 1 : G;
     c.me = tail ? rank - 1 : rank;
     const int runs = (lv.g[0].units + own_units(NR) - 1) / own_units(NR);
@@ -926,15 +938,28 @@ Grid grid_of(const MeshDev &m) {
   return g;
 }
 
+// The fraction of the matrix values that stays in L2 at the normal priority, the others being the first to go: what
+// three fifths of it hold.  Streamed all alike, values that exceed the L2 push each other out before the next pass reads
+// them, and the vectors with them: 8 x 30^3 damage 14.1 ms, and 13.6 so (13.75 with 0.85 of the L2), 60^3 14.4 and 14.0.
+float keep_fraction(double bytes) {
+  int dev = 0, l2 = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 1.f;
+  }
+  const double f = 0.6 * l2 / bytes;
+  return f < 1.0 ? (float)f : 1.f;
+}
+
 template <int NR, bool MG>
 int launch(const Levels &lv, const Inst *insts, const int *list, int nlist, int G, const double *rel_tols,
-           double abs_tol, int max_its, int pairs, cudaStream_t s) {
+           double abs_tol, int max_its, int pairs, float keep, cudaStream_t s) {
   Levels l = lv;
   const size_t smem = kCtxBytes + kHeldFloats * sizeof(float);
   const void *f = (const void *)k_coop_cg32<NR, MG>;
   cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  void *args[] = {&l, &insts, &list, &G, &rel_tols, &abs_tol, &max_its, &pairs};
+  void *args[] = {&l, &insts, &list, &G, &rel_tols, &abs_tol, &max_its, &pairs, &keep};
   e = cudaLaunchCooperativeKernel(f, dim3(nlist * G), dim3(kThreads), args, smem, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
@@ -979,9 +1004,10 @@ int mgb_launch_coop_cg32(const MeshDev *levels, int nlevels, const Inst *insts, 
   const int per = nr == 1 ? 1 : kGroups / own_units(6), most = (runs + per - 1) / per + (lv.tail < nlevels ? 1 : 0);
   if (G > most) G = most;
   const bool mg = nlevels > 1;
+  const float keep = keep_fraction((double)kEllPerNode * sizeof(float) * levels[0].np * nlist);
 #define MGB_COOP(NR)                                                                                                  \
-  (mg ? launch<NR, true>(lv, insts, list, nlist, G, rel_tols, abs_tol, max_its, pairs, s)                     \
-      : launch<NR, false>(lv, insts, list, nlist, G, rel_tols, abs_tol, max_its, pairs, s))
+  (mg ? launch<NR, true>(lv, insts, list, nlist, G, rel_tols, abs_tol, max_its, pairs, keep, s)                     \
+      : launch<NR, false>(lv, insts, list, nlist, G, rel_tols, abs_tol, max_its, pairs, keep, s))
   return nr == 1 ? MGB_COOP(1) : MGB_COOP(6);
 #undef MGB_COOP
 }
