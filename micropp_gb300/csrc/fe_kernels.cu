@@ -585,14 +585,15 @@ constexpr int kAsmRow = kEllPerNode + 2;  // 245 floats: odd stride, conflict-fr
 __host__ __device__ constexpr int corner_x(int b) { return ((b & 3) == 1 || (b & 3) == 2) ? 1 : 0; }
 __host__ __device__ constexpr int corner_y(int b) { return (b & 3) >= 2 ? 1 : 0; }
 __host__ __device__ constexpr int corner_z(int b) { return b >> 2; }
-__host__ __device__ constexpr int local_c(int ox, int oy, int oz) { return oz * 4 + (oy ? 3 - ox : ox); }
 // Stencil slot (0..26) of the neighbour at offset (dx,dy,dz).
 __host__ __device__ constexpr int slot_of(int dx, int dy, int dz) { return (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1); }
 
-template <int EP, int B>
-__device__ __forceinline__ void asm_add_b(float (&acc)[8][9], float A, float cw, const float (&va)[3],
-                                          const float *dg, const float (&s)[6], const float *__restrict__ K) {
-  constexpr int a = local_c(1 - (EP & 1), 1 - ((EP >> 1) & 1), 1 - (EP >> 2));
+// The 8 warps of a block run the same code, their local corner a a number: a copy of it per corner (the corner a
+// constant, the addresses immediate) does not fit in the instruction cache, and 9.4 of the 17 cycles between a warp's
+// instructions were waits for it.  32 x 60^3: 19.0 ms with the copies, 9.7 so.
+template <int B>
+__device__ __forceinline__ void asm_add_b(float (&acc)[8][9], float A, float cw, const float (&va)[3], const float *dg,
+                                          const float (&s)[6], const float *__restrict__ K) {
   const float gx = dg[B * 3], gy = dg[B * 3 + 1], gz = dg[B * 3 + 2];
   const float vb[3] = {gx * s[0] + gy * s[3] + gz * s[4], gy * s[1] + gx * s[3] + gz * s[5],
                        gz * s[2] + gx * s[4] + gy * s[5]};
@@ -600,32 +601,24 @@ __device__ __forceinline__ void asm_add_b(float (&acc)[8][9], float A, float cw,
   for (int fi = 0; fi < 3; ++fi)
 #pragma unroll
     for (int fj = 0; fj < 3; ++fj)
-      acc[B][fi * 3 + fj] += A * __ldg(&K[(a * 3 + fi) * 24 + B * 3 + fj]) + cw * va[fi] * vb[fj];
+      acc[B][fi * 3 + fj] += A * __ldg(&K[fi * 24 + B * 3 + fj]) + cw * va[fi] * vb[fj];
 }
 
-template <int EP, int B>
-__device__ __forceinline__ void asm_add_b_elastic(float (&acc)[8][9], const float *__restrict__ K) {
-  constexpr int a = local_c(1 - (EP & 1), 1 - ((EP >> 1) & 1), 1 - (EP >> 2));
-#pragma unroll
-  for (int q = 0; q < 9; ++q) acc[B][q] += __ldg(&K[(a * 3 + q / 3) * 24 + B * 3 + q % 3]);
-}
-
-template <int EP>
+// acc = the blocks of the element at position ep around node (i, j, k), in which it is corner a
 __device__ __forceinline__ void asm_ep(const MeshDev &m, const Mats &mats, const int8_t *__restrict__ etype,
-                                           const float *__restrict__ k0g, const float *__restrict__ kesum,
-                                           const float *dsh, const float *__restrict__ gpd, int i, int j, int k,
-                                           float (&acc)[8][9]) {
-  constexpr int a = local_c(1 - (EP & 1), 1 - ((EP >> 1) & 1), 1 - (EP >> 2));
-  const int ex = i - 1 + (EP & 1), ey = j - 1 + ((EP >> 1) & 1), ez = k - 1 + (EP >> 2);
+                                       const float *__restrict__ k0g, const float *__restrict__ kesum, const float *dsh,
+                                       const float *__restrict__ gpd, int i, int j, int k, int ep, int a,
+                                       float (&acc)[8][9]) {
+  const int ex = i - 1 + (ep & 1), ey = j - 1 + ((ep >> 1) & 1), ez = k - 1 + (ep >> 2);
   if (ex < 0 || ey < 0 || ez < 0 || ex >= m.nex || ey >= m.ney || ez >= m.nez) return;
   const int e = (ez * m.ney + ey) * m.nex + ex;
   const int ph = etype[e];
   if (mats.m[ph].type == 0) {
-    const float *K = kesum + ph * 576;
-    asm_add_b_elastic<EP, 0>(acc, K); asm_add_b_elastic<EP, 1>(acc, K);
-    asm_add_b_elastic<EP, 2>(acc, K); asm_add_b_elastic<EP, 3>(acc, K);
-    asm_add_b_elastic<EP, 4>(acc, K); asm_add_b_elastic<EP, 5>(acc, K);
-    asm_add_b_elastic<EP, 6>(acc, K); asm_add_b_elastic<EP, 7>(acc, K);
+    const float *K = kesum + ph * 576 + a * 72;
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+#pragma unroll
+      for (int q = 0; q < 9; ++q) acc[b][q] += __ldg(&K[q / 3 * 24 + b * 3 + q % 3]);
     return;
   }
   const size_t st = (size_t)8 * m.nelem;
@@ -641,36 +634,17 @@ __device__ __forceinline__ void asm_ep(const MeshDev &m, const Mats &mats, const
     const float gx = dg[a * 3], gy = dg[a * 3 + 1], gz = dg[a * 3 + 2];
     const float va[3] = {gx * s[0] + gy * s[3] + gz * s[4], gy * s[1] + gx * s[3] + gz * s[5],
                          gz * s[2] + gx * s[4] + gy * s[5]};
-    const float *K = k0g + ((size_t)ph * 8 + g) * 576;
-    asm_add_b<EP, 0>(acc, A, cw, va, dg, s, K); asm_add_b<EP, 1>(acc, A, cw, va, dg, s, K);
-    asm_add_b<EP, 2>(acc, A, cw, va, dg, s, K); asm_add_b<EP, 3>(acc, A, cw, va, dg, s, K);
-    asm_add_b<EP, 4>(acc, A, cw, va, dg, s, K); asm_add_b<EP, 5>(acc, A, cw, va, dg, s, K);
-    asm_add_b<EP, 6>(acc, A, cw, va, dg, s, K); asm_add_b<EP, 7>(acc, A, cw, va, dg, s, K);
+    const float *K = k0g + ((size_t)ph * 8 + g) * 576 + a * 72;
+    asm_add_b<0>(acc, A, cw, va, dg, s, K);
+    asm_add_b<1>(acc, A, cw, va, dg, s, K);
+    asm_add_b<2>(acc, A, cw, va, dg, s, K);
+    asm_add_b<3>(acc, A, cw, va, dg, s, K);
+    asm_add_b<4>(acc, A, cw, va, dg, s, K);
+    asm_add_b<5>(acc, A, cw, va, dg, s, K);
+    asm_add_b<6>(acc, A, cw, va, dg, s, K);
+    asm_add_b<7>(acc, A, cw, va, dg, s, K);
   }
 }
-
-template <int EP>
-__device__ __forceinline__ void asm_store(const float (&acc)[8][9], float *row) {
-  constexpr int a = local_c(1 - (EP & 1), 1 - ((EP >> 1) & 1), 1 - (EP >> 2));
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const int sl = slot_of(corner_x(b) - corner_x(a), corner_y(b) - corner_y(a), corner_z(b) - corner_z(a));
-#pragma unroll
-    for (int q = 0; q < 9; ++q) row[sl * 9 + q] += acc[b][q];
-  }
-}
-
-#define MGB_EP_SWITCH(w, CALL) \
-  switch (w) {                 \
-    case 0: CALL(0); break;    \
-    case 1: CALL(1); break;    \
-    case 2: CALL(2); break;    \
-    case 3: CALL(3); break;    \
-    case 4: CALL(4); break;    \
-    case 5: CALL(5); break;    \
-    case 6: CALL(6); break;    \
-    default: CALL(7); break;   \
-  }
 
 __global__ void __launch_bounds__(kAsmNodes * 8) k_asm_gather32(MeshDev m, Mats mats, const int8_t *etype,
                                                               const float *k0g, const float *kesum,
@@ -692,18 +666,17 @@ __global__ void __launch_bounds__(kAsmNodes * 8) k_asm_gather32(MeshDev m, Mats 
   for (int b = 0; b < 8; ++b)
 #pragma unroll
     for (int q = 0; q < 9; ++q) acc[b][q] = 0.f;
-  if (valid) {
-#define MGB_ASM_CALL(E) asm_ep<E>(m, mats, etype, k0g, kesum, dsh, I.gpd, i, j, k, acc)
-    MGB_EP_SWITCH(w, MGB_ASM_CALL)
-#undef MGB_ASM_CALL
-  }
+  const int ax = 1 - (w & 1), ay = 1 - ((w >> 1) & 1), az = 1 - (w >> 2);  // the node's corner of this warp's element
+  if (valid) asm_ep(m, mats, etype, k0g, kesum, dsh, I.gpd, i, j, k, w, local_of(ax, ay, az), acc);
   // element positions add into the node rows one after the other (fixed summation order)
   for (int p = 0; p < 8; ++p) {
     __syncthreads();
     if (w == p && valid) {
-#define MGB_STORE_CALL(E) asm_store<E>(acc, &rows[lane * kAsmRow])
-      MGB_EP_SWITCH(w, MGB_STORE_CALL)
-#undef MGB_STORE_CALL
+      float *row = &rows[lane * kAsmRow + slot_of(-ax, -ay, -az) * 9];
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) row[(corner_z(b) * 9 + corner_y(b) * 3 + corner_x(b)) * 9 + q] += acc[b][q];
     }
   }
   __syncthreads();
