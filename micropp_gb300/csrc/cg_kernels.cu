@@ -264,7 +264,8 @@ __device__ __forceinline__ double sum8(const double *s, int nblocks) {
   return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
 }
 
-// KMAX: units a block works on at a time, at most.
+// KMAX: units a block works on at a time, at most; the fewer, the more of a row's loads are in registers ahead of its
+// chain of products (20^3 nodes, two units: 18.4 us per iteration with a third of them, 18.0 with all).
 template <int KMAX>
 __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
     k_cg_solve(MeshDev m, const Inst *insts, const int *list, int nlist, int G) {
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
             y = p[fi * np + n];
           } else {
             const double *v = vals + (size_t)(fi * 3) * np + n;
-#pragma unroll(KMAX > 4 ? 3 : 9)
+#pragma unroll(KMAX > 4 ? 3 : 27)
             for (int s = 0; s < 27; ++s) {
               const int nb = n + (s / 9 - 1) * m.nxny + ((s / 3) % 3 - 1) * m.nx + (s % 3 - 1);
               const double *vs = v + (size_t)(s * 9) * np;
@@ -493,7 +494,9 @@ int mgb_launch_cg_solve(const MeshDev *m, const Inst *insts, const int *list, in
   const int K = cdiv(units, G) < 8 ? (int)cdiv(units, G) : 8;
   MeshDev mesh = *m;
   void *args[] = {&mesh, &insts, &list, &nlist, &G};
-  const void *f = K > 4 ? (const void *)k_cg_solve<8> : (const void *)k_cg_solve<4>;
+  const void *f = K > 4   ? (const void *)k_cg_solve<8>
+                  : K > 2 ? (const void *)k_cg_solve<4>
+                          : (const void *)k_cg_solve<2>;
   const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(groups * G), dim3(kUnitThreads * K), args, 0, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();

@@ -53,7 +53,7 @@ constexpr int kMgCoarsePairs = 4;
 constexpr int kMgChunk = 4;
 constexpr int kMgMaxIts = 100;
 
-constexpr size_t kRingBytes = (size_t)64 << 20;
+constexpr size_t kRingBytes = (size_t)96 << 20;
 
 // A structured grid of nx x ny x nz nodes (the multigrid levels and the separable product's intermediates).
 static MeshDev grid_of(int nx, int ny, int nz) {
@@ -498,7 +498,7 @@ double Engine::slot_bytes() const {
 }
 
 // The ring of element matrices that an assembly of n instances works through: two element layers at least, as many as
-// kRingBytes hold beyond that (half of the L2), no more than there are.
+// kRingBytes hold beyond that (three quarters of the L2), no more than there are.
 void Engine::ensure_ring(int n, size_t value_bytes) {
   const size_t layer = (size_t)n * 576 * mesh_.nex * mesh_.ney * value_bytes;
   const size_t bytes = std::max(2 * layer, std::min((mesh_.nez + 1) * layer, kRingBytes));
