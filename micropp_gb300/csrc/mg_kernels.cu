@@ -109,32 +109,43 @@ __device__ __forceinline__ LvView view(const Inst &I, int l) {
 // which: 0 = x, 1 = y, 2 = t
 __device__ __forceinline__ float *pick(const LvView &v, int which) { return which == 0 ? v.x : which == 1 ? v.y : v.t; }
 
-// y = A x at interior node n for NR right-hand sides (slot order, then column order, as the CG SpMVs).
+// y = A x at interior node n for NR right-hand sides (slot order, then column order, as the CG SpMVs).  On the coarse
+// levels a pass is a thread's chain of loads, so kBatch slots' loads go out before their products; on level 0 (STREAM)
+// the warps in flight cover them.
 template <int NR, bool RM, bool STREAM>
 __device__ __forceinline__ void apply_node(const MeshDev &m, const float *__restrict__ vals,
                                            const float *__restrict__ x, int n, float (&y)[NR * 3]) {
+  constexpr int kBatch = STREAM ? 1 : NR == 1 ? 9 : 3;
   const size_t np = m.np;
 #pragma unroll
   for (int c = 0; c < NR * 3; ++c) y[c] = 0.f;
-#pragma unroll 3
-  for (int s = 0; s < 27; ++s) {
-    const int nb = n + (s / 9 - 1) * m.nxny + ((s / 3) % 3 - 1) * m.nx + (s % 3 - 1);
-    float K[9];
+#pragma unroll(STREAM ? 3 : 1)
+  for (int s0 = 0; s0 < 27; s0 += kBatch) {
+    float K[kBatch][9], xv[kBatch][NR * 3];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      const float *a = vals + (size_t)(s * 9 + q) * np + n;
-      K[q] = STREAM ? __ldcs(a) : __ldg(a);
+    for (int h = 0; h < kBatch; ++h) {
+      const int s = s0 + h;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const float *a = vals + (size_t)(s * 9 + q) * np + n;
+        K[h][q] = STREAM ? __ldcs(a) : __ldg(a);
+      }
     }
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      float xv[3];
+    for (int h = 0; h < kBatch; ++h) {
+      const int s = s0 + h, nb = n + (s / 9 - 1) * m.nxny + ((s / 3) % 3 - 1) * m.nx + (s % 3 - 1);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) xv[d] = x[vix<RM>(r, d, nb, np)];
-#pragma unroll
-      for (int fi = 0; fi < 3; ++fi)
-#pragma unroll
-        for (int fj = 0; fj < 3; ++fj) y[r * 3 + fi] = fmaf(K[fi * 3 + fj], xv[fj], y[r * 3 + fi]);
+      for (int c = 0; c < NR * 3; ++c) xv[h][c] = x[vix<RM>(c / 3, c % 3, nb, np)];
     }
+#pragma unroll
+    for (int h = 0; h < kBatch; ++h)
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+#pragma unroll
+        for (int fi = 0; fi < 3; ++fi)
+#pragma unroll
+          for (int fj = 0; fj < 3; ++fj)
+            y[r * 3 + fi] = fmaf(K[h][fi * 3 + fj], xv[h][r * 3 + fj], y[r * 3 + fi]);
   }
 }
 
@@ -246,14 +257,18 @@ __global__ void __launch_bounds__(kMgBlock) k_mg_sdiag(MeshDev m, const Inst *in
   const size_t np = m.np;
   float l1[3] = {0.f, 0.f, 0.f};
 #pragma unroll 1
-  for (int s = 0; s < 27; ++s) {
-    const int nb = n + (s / 9 - 1) * m.nxny + ((s / 3) % 3 - 1) * m.nx + (s % 3 - 1);
-    int bi, bj, bk;
-    if (on_boundary(m, nb, bi, bj, bk)) continue;
+  for (int s0 = 0; s0 < 27; s0 += 9) {
+    float a[81];  // a plane's values go out together
 #pragma unroll
-    for (int fi = 0; fi < 3; ++fi)
+    for (int q = 0; q < 81; ++q) a[q] = vals[(size_t)(s0 * 9 + q) * np + n];
 #pragma unroll
-      for (int fj = 0; fj < 3; ++fj) l1[fi] += fabsf(vals[(size_t)(s * 9 + fi * 3 + fj) * np + n]);
+    for (int h = 0; h < 9; ++h) {
+      // a boundary column adds +0, which changes no sum
+      const int bi = i + h % 3 - 1, bj = j + h / 3 - 1, bk = k + s0 / 9 - 1;
+      const bool in = bi > 0 && bj > 0 && bk > 0 && bi < m.nx - 1 && bj < m.ny - 1 && bk < m.nz - 1;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) l1[q / 3] += in ? fabsf(a[h * 9 + q]) : 0.f;
+    }
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -317,14 +332,20 @@ __global__ void __launch_bounds__(kMgBlock) k_mg_restrict(MeshDev mf, MeshDev mc
 #pragma unroll
   for (int c = 0; c < NR * 3; ++c) acc[c] = 0.f;
 #pragma unroll 1
-  for (int a = 0; a < 27; ++a) {
-    const int ax = a % 3 - 1, ay = (a / 3) % 3 - 1, az = a / 9 - 1;
-    const int i = ((2 * Z + az) * mf.ny + (2 * Y + ay)) * mf.nx + (2 * X + ax);
-    const float w = half_pow(ax) * half_pow(ay) * half_pow(az);
+  for (int az = -1; az <= 1; ++az) {
+    float v[9][NR * 3];  // a plane's values go out together
 #pragma unroll
-    for (int r = 0; r < NR; ++r)
+    for (int a = 0; a < 9; ++a) {
+      const int i = ((2 * Z + az) * mf.ny + (2 * Y + a / 3 - 1)) * mf.nx + (2 * X + a % 3 - 1);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) acc[r * 3 + d] = fmaf(w, f.t[vix<RMF>(r, d, i, npf)], acc[r * 3 + d]);
+      for (int c = 0; c < NR * 3; ++c) v[a][c] = f.t[vix<RMF>(c / 3, c % 3, i, npf)];
+    }
+#pragma unroll
+    for (int a = 0; a < 9; ++a) {
+      const float w = half_pow(a % 3 - 1) * half_pow(a / 3 - 1) * half_pow(az);
+#pragma unroll
+      for (int c = 0; c < NR * 3; ++c) acc[c] = fmaf(w, v[a][c], acc[c]);
+    }
   }
   float kd[3];
 #pragma unroll
@@ -358,23 +379,23 @@ __global__ void __launch_bounds__(kMgBlock) k_mg_prolong(MeshDev mf, MeshDev mc,
       for (int d = 0; d < 3; ++d) f.t[vix<RMF>(r, d, n, npf)] = 0.f;
     return;
   }
-  // coarse parents along each axis: even index -> (i / 2, 1); odd -> ((i - 1) / 2, 1/2), ((i + 1) / 2, 1/2)
-  const int px0 = i >> 1, px1 = (i + 1) >> 1, py0 = j >> 1, py1 = (j + 1) >> 1, pz0 = k >> 1, pz1 = (k + 1) >> 1;
-  const float wx = (i & 1) ? 0.5f : 1.f, wy = (j & 1) ? 0.5f : 1.f, wz = (k & 1) ? 0.5f : 1.f;
-  const int nxo = (i & 1) ? 2 : 1, nyo = (j & 1) ? 2 : 1, nzo = (k & 1) ? 2 : 1;
+  // coarse parents along each axis: even index -> (i / 2, 1); odd -> ((i - 1) / 2, 1/2), ((i + 1) / 2, 1/2).  The loads of
+  // all 8 go out together; an even coordinate's second parent is its first again, and unused.
+  const int oi = i & 1, oj = j & 1, ok = k & 1;
+  const float w = (oi ? 0.5f : 1.f) * (oj ? 0.5f : 1.f) * (ok ? 0.5f : 1.f);
+  const int J0 = ((k >> 1) * mc.ny + (j >> 1)) * mc.nx + (i >> 1);
   float acc[NR * 3];
 #pragma unroll
-  for (int r = 0; r < NR; ++r)
+  for (int c = 0; c < NR * 3; ++c) {
+    const float *xq = xc + (size_t)c * npc + J0;
+    float v[8], x = f.x[vix<RMF>(c / 3, c % 3, n, npf)];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) acc[r * 3 + d] = f.x[vix<RMF>(r, d, n, npf)];
-  for (int cz = 0; cz < nzo; ++cz)
-    for (int cy = 0; cy < nyo; ++cy)
-      for (int cx = 0; cx < nxo; ++cx) {
-        const int J = ((cz ? pz1 : pz0) * mc.ny + (cy ? py1 : py0)) * mc.nx + (cx ? px1 : px0);
-        const float w = wx * wy * wz;
+    for (int q = 0; q < 8; ++q) v[q] = xq[(ok & (q >> 2)) * mc.nxny + (oj & (q >> 1)) * mc.nx + (oi & q)];
 #pragma unroll
-        for (int c = 0; c < NR * 3; ++c) acc[c] = fmaf(w, xc[(size_t)c * npc + J], acc[c]);
-      }
+    for (int q = 0; q < 8; ++q)
+      if ((q & 1) <= oi && ((q >> 1) & 1) <= oj && (q >> 2) <= ok) x = fmaf(w, v[q], x);
+    acc[c] = x;
+  }
 #pragma unroll
   for (int r = 0; r < NR; ++r)
 #pragma unroll
