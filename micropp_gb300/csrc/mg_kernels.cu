@@ -189,17 +189,20 @@ __device__ __forceinline__ void apply_node_h(const MeshDev &m, const unsigned sh
 // fixed.  src / dst: 0 = level lf's operator, 1 = mid1, 2 = mid2, 3 = level lf + 1's operator.
 __global__ void __launch_bounds__(kMgBlock) k_mg_rap1(MeshDev mi, MeshDev mo, const Inst *insts, const int *list,
                                                       int lf, int axis, int src, int dst) {
-  const Inst &I = insts[list[blockIdx.y]];
+  const Inst &I = insts[list[blockIdx.z]];
   const MgInst &G = *I.mg;
   const float *__restrict__ A = src == 0 ? (lf == 0 ? I.vals32 : G.lv[lf].vals) : src == 1 ? G.mid1 : G.mid2;
   float *__restrict__ B = dst == 3 ? G.lv[lf + 1].vals : dst == 1 ? G.mid1 : G.mid2;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 27 * mo.nn) return;
-  const int S = t / mo.nn, io = t - S * mo.nn;
-  int c[3] = {io % mo.nx, (io / mo.nx) % mo.ny, io / mo.nxny};
+  // S is the block's, so which terms there are is too; blocks that follow one another differ along the axis, whose three
+  // offsets read the same three input blocks of a node
+  const int third = blockIdx.y % 3, rest = blockIdx.y / 3;
+  const int S = axis == 0 ? blockIdx.y : axis == 1 ? rest / 3 * 9 + third * 3 + rest % 3 : third * 9 + rest;
+  const int io = blockIdx.x * blockDim.x + threadIdx.x;
+  if (io >= mo.nn) return;
+  const int c[3] = {io % mo.nx, (io / mo.nx) % mo.ny, io / mo.nxny};
   const int so[3] = {S % 3 - 1, (S / 3) % 3 - 1, S / 9 - 1};
-  const int dimo[3] = {mo.nx, mo.ny, mo.nz}, dimi[3] = {mi.nx, mi.ny, mi.nz};
-  const int X = c[axis], JX = X + so[axis];
+  const int dimo[3] = {mo.nx, mo.ny, mo.nz}, dimi = axis == 0 ? mi.nx : axis == 1 ? mi.ny : mi.nz;
+  const int sa = so[axis], X = c[axis], JX = X + sa;
   bool live = X > 0 && X < dimo[axis] - 1 && JX > 0 && JX < dimo[axis] - 1;
 #pragma unroll
   for (int d = 0; d < 3; ++d)
@@ -209,23 +212,27 @@ __global__ void __launch_bounds__(kMgBlock) k_mg_rap1(MeshDev mi, MeshDev mo, co
   for (int q = 0; q < 9; ++q) acc[q] = 0.f;
   if (live) {
     const size_t npi = mi.np;
+    const int along = axis == 0 ? 1 : axis == 1 ? mi.nx : mi.nxny, slot = axis == 0 ? 1 : axis == 1 ? 3 : 9;
+    const int i0 = (c[0] << (axis == 0)) + mi.nx * (c[1] << (axis == 1)) + mi.nxny * (c[2] << (axis == 2));
 #pragma unroll
     for (int a = -1; a <= 1; ++a) {
       const int ix = 2 * X + a;
-      if (ix <= 0 || ix >= dimi[axis] - 1) continue;
-      int f[3] = {c[0], c[1], c[2]};
-      f[axis] = ix;
-      const int i = f[0] + mi.nx * (f[1] + mi.ny * f[2]);
+      float v[3][9];
 #pragma unroll
       for (int o = -1; o <= 1; ++o) {
-        const int jx = ix + o, e = jx - 2 * JX;
-        if (e < -1 || e > 1 || jx <= 0 || jx >= dimi[axis] - 1) continue;
-        int off[3] = {so[0], so[1], so[2]};
-        off[axis] = o;
-        const int sf = (off[2] + 1) * 9 + (off[1] + 1) * 3 + (off[0] + 1);
+        const int e = a + o - 2 * sa;
+        if (e < -1 || e > 1) continue;
+        const float *__restrict__ src_o = A + (size_t)((S + (o - sa) * slot) * 9) * npi + (i0 + a * along);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) v[o + 1][q] = __ldg(src_o + q * npi);
+      }
+#pragma unroll
+      for (int o = -1; o <= 1; ++o) {
+        const int e = a + o - 2 * sa, jx = ix + o;
+        if (e < -1 || e > 1 || ix <= 0 || ix >= dimi - 1 || jx <= 0 || jx >= dimi - 1) continue;
         const float w = half_pow(a) * half_pow(e);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) acc[q] = fmaf(w, __ldg(A + (size_t)(sf * 9 + q) * npi + i), acc[q]);
+        for (int q = 0; q < 9; ++q) acc[q] = fmaf(w, v[o + 1][q], acc[q]);
       }
     }
   }
@@ -811,8 +818,7 @@ int mgb_launch_mg_rap1(const MeshDev *mi, const MeshDev *mo, const Inst *insts, 
                        int axis, int src, int dst, cudaStream_t s) {
   if (nlist <= 0) return 0;
   if (axis < 0 || axis > 2 || src < 0 || src > 2 || dst < 1 || dst > 3 || src == dst) return (int)cudaErrorInvalidValue;
-  k_mg_rap1<<<dim3(cdiv((size_t)27 * mo->nn, kMgBlock), nlist), kMgBlock, 0, s>>>(*mi, *mo, insts, list, lf, axis, src,
-                                                                               dst);
+  k_mg_rap1<<<dim3(cdiv(mo->nn, kMgBlock), 27, nlist), kMgBlock, 0, s>>>(*mi, *mo, insts, list, lf, axis, src, dst);
   return (int)cudaGetLastError();
 }
 
