@@ -53,6 +53,7 @@ constexpr int kMgCoarsePairs = 4;
 constexpr int kMgChunk = 4;
 constexpr int kMgMaxIts = 100;
 
+constexpr size_t kLists = 32;
 constexpr size_t kRingBytes = (size_t)96 << 20;
 
 // A structured grid of nx x ny x nz nodes (the multigrid levels and the separable product's intermediates).
@@ -533,7 +534,6 @@ void Engine::ensure_slots(int n) {
     w.red = dalloc<double>((size_t)nblocks * kRedStride, "partials");
     w.ticket = dalloc<unsigned int>(1, "ticket");
     w.cg = dalloc<CgState>(1, "cg state");
-    w.out = dalloc<InstOut>(1, "out");
     if (fp64) {
       w.r = dalloc<double>(nd, "r");
       w.z = dalloc<double>((size_t)3 * mesh_.np, "z");
@@ -604,9 +604,14 @@ void Engine::ensure_slots(int n) {
       check(cudaMemcpy(w.mg, &h, sizeof(MgInst), cudaMemcpyHostToDevice), "multigrid hierarchy upload");
     }
     check(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned int), stream_), "ticket");
-    check(cudaMemsetAsync(w.out, 0, sizeof(InstOut), stream_), "out");
   }
   clear_graphs();  // the captured chunks hold the instance and list pointers
+  // the slots' outputs lie side by side: one copy brings them all back
+  dfree(d_outs_);
+  d_outs_ = nullptr;
+  d_outs_ = dalloc<InstOut>(n, "out");
+  check(cudaMemsetAsync(d_outs_, 0, n * sizeof(InstOut), stream_), "out");
+  for (int s = 0; s < n; ++s) slots_[s].out = d_outs_ + s;
   dfree(d_insts_);
   d_insts_ = dalloc<Inst>(n, "insts");
   if (eta_cap_ < n) {
@@ -637,6 +642,12 @@ void Engine::ensure_slots(int n) {
     dfree(d_list_);
     d_list_ = dalloc<int>(n, "list");
     list_cap_ = n;
+    sync();
+    if (h_list_) cudaFreeHost(h_list_);
+    h_list_ = nullptr;
+    h_list_cap_ = 0;
+    check(cudaMallocHost((void **)&h_list_, kLists * n * sizeof(int)), "pinned list");
+    h_list_cap_ = kLists * n;
   }
 }
 
@@ -654,14 +665,18 @@ void Engine::free_slots() {
     dfree(w.ticket);
     dfree(w.cg);
     dfree(w.cg6);
-    dfree(w.out);
   }
   slots_.clear();
+  dfree(d_outs_);
+  d_outs_ = nullptr;
   dfree(d_insts_);
   d_insts_ = nullptr;
   dfree(d_list_);
   d_list_ = nullptr;
   list_cap_ = 0;
+  if (h_list_) cudaFreeHost(h_list_);
+  h_list_ = nullptr;
+  h_list_cap_ = 0;
   if (h_out_) cudaFreeHost(h_out_);
   h_out_ = nullptr;
 }
@@ -671,23 +686,22 @@ void Engine::upload_insts() {
         "insts upload");
 }
 
+// From pinned memory that holds kLists lists before the stream is waited for (sync() frees it), so that the host goes on.
 void Engine::upload_list(const std::vector<int> &slots) {
-  check(cudaMemcpyAsync(d_list_, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, stream_),
-        "list upload");
-  // The host vector may change right after; wait for the copy of pageable memory to be consumed.
-  check(cudaStreamSynchronize(stream_), "list sync");
+  if (list_used_ + slots.size() > h_list_cap_) sync();
+  int *h = h_list_ + list_used_;
+  std::copy(slots.begin(), slots.end(), h);
+  list_used_ += slots.size();
+  check(cudaMemcpyAsync(d_list_, h, slots.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "list upload");
 }
 
 void Engine::download_out() {
-  for (size_t s = 0; s < slots_.size(); ++s)
-    check(cudaMemcpyAsync(&h_out_[s], slots_[s].out, sizeof(InstOut), cudaMemcpyDeviceToHost, stream_), "out");
+  check(cudaMemcpyAsync(h_out_, d_outs_, slots_.size() * sizeof(InstOut), cudaMemcpyDeviceToHost, stream_), "out");
   sync();
   for (size_t s = 0; s < slots_.size(); ++s)
     if (h_out_[s].stalled) {
-      for (Slot &w : slots_) {
-        cudaMemsetAsync(w.ticket, 0, sizeof(unsigned int), stream_);
-        cudaMemsetAsync(w.out, 0, sizeof(InstOut), stream_);
-      }
+      for (Slot &w : slots_) cudaMemsetAsync(w.ticket, 0, sizeof(unsigned int), stream_);
+      cudaMemsetAsync(d_outs_, 0, slots_.size() * sizeof(InstOut), stream_);
       throw std::runtime_error("a linear solve stalled: a block of its launch never arrived");
     }
 }
@@ -699,7 +713,10 @@ double Engine::listed_cg_its(const std::vector<int> &slots) {
   return its;
 }
 
-void Engine::sync() { check(cudaStreamSynchronize(stream_), "stream synchronize"); }
+void Engine::sync() {
+  check(cudaStreamSynchronize(stream_), "stream synchronize");
+  list_used_ = 0;
+}
 
 // A chunk of CG iterations (`body` launches them on stream_): replayed from a CUDA graph captured the first
 // time this (solver, batch size) pair runs, or launched directly while per-kernel timing is on or graphs are
@@ -892,13 +909,7 @@ void Engine::residual(const std::vector<int> &slots) {
 // ell_solve_cgpd for the listed slots (b -> du); out.cg_its of each slot is valid afterwards.
 void Engine::cg_solve(const std::vector<int> &slots) {
   const int n = (int)slots.size();
-  for (int s : slots) {
-    CgState c{};
-    c.min_err = cg_abs_tol_;
-    c.rel_err = cg_rel_tol_;
-    c.max_its = cg_max_its_;
-    check(cudaMemcpyAsync(slots_[s].cg, &c, sizeof(CgState), cudaMemcpyHostToDevice, stream_), "cg init");
-  }
+  cg_init(std::vector<double>(n, cg_rel_tol_), cg_max_its_);
   launches_ += 2;
   check_launch(mgb_launch_cg_setup(&mesh_, d_insts_, d_list_, n, stream_), "cg setup");
   // Algorithmic bytes per iteration and RVE (spmv): 81 values per row + x read + y written.
@@ -944,6 +955,15 @@ void Engine::cg_solve(const std::vector<int> &slots) {
   }
 }
 
+// The CG states of the listed instances at the start of a solve, their relative tolerances also in d_eta_.
+void Engine::cg_init(const std::vector<double> &rel_tols, int max_its) {
+  const int n = (int)rel_tols.size();
+  std::copy(rel_tols.begin(), rel_tols.end(), h_eta_);
+  check(cudaMemcpyAsync(d_eta_, h_eta_, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "CG tolerances");
+  launches_ += 1;
+  check_launch(mgb_launch_cg32_init(d_insts_, d_list_, n, d_eta_, cg_abs_tol_, max_its, stream_), "cg init");
+}
+
 // Whether an FP32 solve of n listed instances runs in one cooperative launch: batches small enough, unless
 // per-kernel timers want the iterations launched kernel by kernel or the V-cycle reads the FP16 operator.
 bool Engine::coop32(int n, bool use_mg) const {
@@ -969,18 +989,8 @@ bool Engine::coop_solve32(int n, int nr, bool use_mg) {
 void Engine::cg_solve32(const std::vector<int> &slots, const std::vector<double> &rel_tols, bool use_mg) {
   const int n = (int)slots.size();
   const bool mg = mg_ && use_mg;
-  if (coop32(n, use_mg)) {
-    for (int a = 0; a < n; ++a) h_eta_[a] = rel_tols[a];
-    check(cudaMemcpyAsync(d_eta_, h_eta_, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "CG tolerances");
-    if (coop_solve32(n, 1, use_mg)) return;
-  }
-  for (int a = 0; a < n; ++a) {
-    CgState c{};
-    c.min_err = cg_abs_tol_;
-    c.rel_err = rel_tols[a];
-    c.max_its = mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_;
-    check(cudaMemcpyAsync(slots_[slots[a]].cg, &c, sizeof(CgState), cudaMemcpyHostToDevice, stream_), "cg init");
-  }
+  cg_init(rel_tols, mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_);
+  if (coop32(n, use_mg) && coop_solve32(n, 1, use_mg)) return;
   launches_ += 1;
   check_launch(mgb_launch_cg32_setup(&mesh_, d_insts_, d_list_, n, mg ? 1 : 0, stream_), "cg32 setup");
   if (mg) mg_vcycle(1, n, true, 128);
@@ -1164,6 +1174,7 @@ std::vector<int> Engine::tangent_solve(const std::vector<int> &slots, bool use_m
   const bool energy = gather32_;
   const double sweep_rel = energy ? kTangentSweepRelEnergy : kTangentSweepRel;
   const double tangent_tol = energy ? kTangentTolEnergy : kTangentTol;
+  const int max_its = mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_;
   std::vector<char> mg_capped(n, 0);  // a multigrid sweep of the slot reached kMgMaxIts
   std::vector<int> its(n, 0);
   upload_insts();
@@ -1183,14 +1194,9 @@ std::vector<int> Engine::tangent_solve(const std::vector<int> &slots, bool use_m
   std::vector<int> live_idx(n);
   for (int i = 0; i < n; ++i) live_idx[i] = i;
   for (int sweep = 0; sweep < kTangentSweeps && !live.empty(); ++sweep) {
-    for (int s : live) {
-      Cg6State c{};
-      c.min_err = 0.0;
-      c.rel_err = sweep_rel;
-      c.max_its = mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_;
-      check(cudaMemcpyAsync(slots_[s].cg6, &c, sizeof(Cg6State), cudaMemcpyHostToDevice, stream_), "cg6 init");
-    }
     if (sweep > 0) upload_list(live);
+    launches_ += 1;
+    check_launch(mgb_launch_cg6_init(d_insts_, d_list_, (int)live.size(), sweep_rel, max_its, stream_), "cg6 init");
     launches_ += 1;
     timer_begin(t_tan_, 0.0);
     check_launch(mgb_launch_t6_residual(&mesh_, d_insts_, d_list_, (int)live.size(), sweep == 0 ? 1 : 0,
@@ -1214,14 +1220,8 @@ std::vector<int> Engine::tangent_solve(const std::vector<int> &slots, bool use_m
       live_idx = next_idx;
       if (live.empty()) break;
       upload_list(live);
-      for (int s : live) {
-        Cg6State c{};
-        c.min_err = 0.0;
-        c.rel_err = sweep_rel;
-        c.max_its = mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_;
-        check(cudaMemcpyAsync(slots_[s].cg6, &c, sizeof(Cg6State), cudaMemcpyHostToDevice, stream_), "cg6 init");
-      }
-      launches_ += 1;
+      launches_ += 2;
+      check_launch(mgb_launch_cg6_init(d_insts_, d_list_, (int)live.size(), sweep_rel, max_its, stream_), "cg6 init");
       timer_begin(t_tan_, 0.0);
       check_launch(mgb_launch_t6_residual(&mesh_, d_insts_, d_list_, (int)live.size(), sweep == 0 ? 1 : 0,
                                           mg ? 1 : 0, stream_),
@@ -1645,6 +1645,7 @@ void Engine::allocate_vars(GpState &g) {
 void Engine::homogenize_fe_batch(const std::vector<int> &gp_ids) {
   const int n = (int)gp_ids.size();
   const size_t ubytes = nndim() * sizeof(double);
+  check(cudaMemsetAsync(d_outs_, 0, n * sizeof(InstOut), stream_), "out reset");
   std::vector<int> all(n);
   for (int i = 0; i < n; ++i) all[i] = i;
   std::vector<std::array<double, 6>> strains(n);
@@ -1657,7 +1658,6 @@ void Engine::homogenize_fe_batch(const std::vector<int> &gp_ids) {
     I.has_vars_old = g.allocated ? 1 : 0;
     I.vars_new = g.allocated ? g.vars_k : w.vars_aux;
     if (!g.allocated) check(cudaMemsetAsync(w.vars_aux, 0, nvars() * sizeof(double), stream_), "vars aux");
-    check(cudaMemsetAsync(w.out, 0, sizeof(InstOut), stream_), "out reset");
     g.cost = 0;
     g.subiterated = false;
     g.status = 0;
@@ -1733,7 +1733,7 @@ void Engine::homogenize_fe_batch(const std::vector<int> &gp_ids) {
   }
 
   // calc_vars_new (update.cpp:32-56) at u_k = the slot's u.
-  for (int i = 0; i < n; ++i) check(cudaMemsetAsync(&slots_[i].out->nonlinear, 0, sizeof(int), stream_), "flag");
+  check(cudaMemset2DAsync(&d_outs_->nonlinear, sizeof(InstOut), 0, sizeof(int), n, stream_), "flag");
   upload_insts();
   upload_list(all);
   launches_ += 1;

@@ -172,6 +172,7 @@ class Engine {
   void residual(const std::vector<int> &slots);
   void cg_solve(const std::vector<int> &slots);
   void ensure_ring(int n, size_t value_bytes);
+  void cg_init(const std::vector<double> &rel_tols, int max_its);
   bool coop32(int n, bool use_mg) const;
   bool coop_solve32(int n, int nr, bool use_mg);
   void cg_solve32(const std::vector<int> &slots, const std::vector<double> &rel_tols, bool use_mg = true);
@@ -268,6 +269,9 @@ class Engine {
   KernelTimer t_rap_;  // multigrid operators after an assembly: smoother diagonals and Galerkin products
   KernelTimer t_tan_;  // FP64 kernels of the implicit ctan: right-hand sides, refinement residuals, ctan sums
   KernelTimer t_mg1_, t_mg6_, t_mgc_;  // V-cycles: level-0 passes (1 and 6 RHS), coarse levels and transfers
+  InstOut *d_outs_ = nullptr;  // the slots' outputs
+  int *h_list_ = nullptr;      // pinned: the lists uploaded since the stream was last waited for
+  size_t h_list_cap_ = 0, list_used_ = 0;
   char *d_ring_ = nullptr;  // element matrices of a few layers (ensure_ring)
   size_t ring_bytes_ = 0;
   PathState path_;

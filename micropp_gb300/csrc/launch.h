@@ -70,6 +70,9 @@ int mgb_launch_add_du32(const mgb::MeshDev *m, const mgb::Inst *insts, const int
 // CG states of the listed instances at the start of a solve, from a device array of relative tolerances.
 int mgb_launch_cg32_init(const mgb::Inst *insts, const int *list, int nlist, const double *rel_tol, double abs_tol,
                          int max_its, cudaStream_t s);
+// The same for the tangent CG (all right-hand sides with one tolerance), before mgb_launch_t6_residual.
+int mgb_launch_cg6_init(const mgb::Inst *insts, const int *list, int nlist, double rel_tol, int max_its,
+                        cudaStream_t s);
 // *p = 0 (a kernel, so that it can sit in a conditional node's body).
 int mgb_launch_zero_u32(unsigned int *p, cudaStream_t s);
 // The condition of a captured CG loop (a WHILE node): continue while *count != 0 and fewer than cap chunks ran.

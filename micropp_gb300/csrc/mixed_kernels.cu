@@ -953,6 +953,16 @@ __global__ void k_cg32_init(const Inst *insts, const int *list, int nlist, const
   *insts[list[a]].cg = c;
 }
 
+// The same for the tangent CG, before mgb_launch_t6_residual.
+__global__ void k_cg6_init(const Inst *insts, const int *list, int nlist, double rel_tol, int max_its) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= nlist) return;
+  Cg6State c{};
+  c.rel_err = rel_tol;
+  c.max_its = max_its;
+  *insts[list[a]].cg6 = c;
+}
+
 __global__ void k_zero_u32(unsigned int *p) { *p = 0u; }
 
 // Condition of the WHILE node of a captured CG solve: another chunk of iterations runs while some instance of
@@ -978,6 +988,12 @@ int mgb_launch_cg32_init(const Inst *insts, const int *list, int nlist, const do
                          int max_its, cudaStream_t s) {
   if (nlist <= 0) return 0;
   k_cg32_init<<<cdiv(nlist, 128), 128, 0, s>>>(insts, list, nlist, rel_tol, abs_tol, max_its);
+  return (int)cudaGetLastError();
+}
+
+int mgb_launch_cg6_init(const Inst *insts, const int *list, int nlist, double rel_tol, int max_its, cudaStream_t s) {
+  if (nlist <= 0) return 0;
+  k_cg6_init<<<cdiv(nlist, 128), 128, 0, s>>>(insts, list, nlist, rel_tol, max_its);
   return (int)cudaGetLastError();
 }
 
