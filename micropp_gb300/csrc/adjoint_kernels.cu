@@ -393,8 +393,11 @@ __global__ void __launch_bounds__(kNodeBlock) k_bicg_r(MeshDev m, AdjDev A, unsi
 // every phase.  A 12^3 J2 path of 4 steps, forward and reverse: 503 ms launched, 171 ms so.
 constexpr int kBicgUnit = 288;  // threads per unit
 constexpr int kBicgGroups = 3;  // units a block works on at a time, at most
-// Largest RVE (nodes) solved in one launch.
-constexpr int kBicgNodes = 100000;
+// Largest RVE (nodes) solved in one launch: the largest it was measured at.  The launched iteration is five kernels and
+// re-reads the vectors between them; a load step and its reverse pass (damage, edges of 6, 12, 20, 30, 45, 60, 75, 90)
+// take 21.6, 38.6, 61.9, 99, 335, 717, 1792, 2864 ms launched and 9.1, 14.3, 26.6, 74, 230, 568, 1408, 2673 in one
+// launch: the gain shrinks to 7% where the vectors outgrow L2.
+constexpr int kBicgNodes = 800000;
 
 template <bool Transpose>
 __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDev m, AdjDev A, int units) {

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kMgBlock) k_mg_rap1(MeshDev mi, MeshDev mo, co
   const MgInst &G = *I.mg;
   const float *__restrict__ A = src == 0 ? (lf == 0 ? I.vals32 : G.lv[lf].vals) : src == 1 ? G.mid1 : G.mid2;
   float *__restrict__ B = dst == 3 ? G.lv[lf + 1].vals : dst == 1 ? G.mid1 : G.mid2;
-  // S is the block's, so which terms there are is too; blocks that follow one another differ along the axis, whose three
+  // S is the block's, so which terms there are is too; blocks that follow one another differ along the axis whose three
   // offsets read the same three input blocks of a node
   const int third = blockIdx.y % 3, rest = blockIdx.y / 3;
   const int S = axis == 0 ? blockIdx.y : axis == 1 ? rest / 3 * 9 + third * 3 + rest % 3 : third * 9 + rest;
@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(kMgBlock) k_mg_prolong(MeshDev mf, MeshDev mc,
       for (int d = 0; d < 3; ++d) f.t[vix<RMF>(r, d, n, npf)] = 0.f;
     return;
   }
-  // coarse parents along each axis: even index -> (i / 2, 1); odd -> ((i - 1) / 2, 1/2), ((i + 1) / 2, 1/2).  The loads of
-  // all 8 go out together; an even coordinate's second parent is its first again, and unused.
+  // coarse parents along each axis: even index -> (i / 2, 1); odd -> ((i - 1) / 2, 1/2), ((i + 1) / 2, 1/2).  All 8
+  // loads go out together; an even coordinate's second parent is its first again, and unused.
   const int oi = i & 1, oj = j & 1, ok = k & 1;
   const float w = (oi ? 0.5f : 1.f) * (oj ? 0.5f : 1.f) * (ok ? 0.5f : 1.f);
   const int J0 = ((k >> 1) * mc.ny + (j >> 1)) * mc.nx + (i >> 1);

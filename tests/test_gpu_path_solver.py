@@ -14,7 +14,7 @@ MATS = ((0, 1e7, 0.25, 0, 0, 0), (0, 1e8, 0.25, 0, 0, 0), (0, 1e7, 0.25, 0, 0, 0
 
 # less than one unit of 32 nodes, remainders, one unit per block, several units per block in turn, and a grid above the
 # size that one launch takes
-@pytest.mark.parametrize("n", [2, (3, 4, 2), (7, 4, 9), 12, 25, 47])
+@pytest.mark.parametrize("n", [2, (3, 4, 2), (7, 4, 9), 12, 25, 47, 94])
 def test_elastic_path_is_the_linear_ctan(gpu_lib, n):
     import micropp_gb300 as mg
     g = mg.Micropp(gpu_config(n, mats=MATS, coupling=[2], lin_stress=0, micro_type=1, geo=(0.2, 0, 0, 0), nr_max_its=4,
