@@ -24,6 +24,9 @@ namespace mgb {
 constexpr int kUpdRows = 4;  // rows per thread of the vector update
 // Largest batch (nodes of all its instances) solved by one cooperative launch: above, the two forms are equal (60^3 nodes)
 // or the launches faster (damage, plain form, 8 x 30^3 179 ms against 186, 32 x 20^3 191 against 210).
+// Handles at work at the same time count as one batch (each as large as the caller's), since their launches overlap: 16
+// points of 30^3, a handle each, 338 ms with every solve in one launch on all SMs, 199 launched.  Below that they share
+// the SMs (AtWork::parts): 16 J2 points of 20^3 3,430 ms on all SMs each, 1,580 so, 1,656 launched; 4 of them 848, 525, 702.
 constexpr long long kSolveNodes = 150000;
 // Microseconds of an iteration in one launch: a block's unit of 32 nodes (243 FP64 warp instructions of 64 cycles on
 // four quarters), the shortest unit (its chain of dependent products), and the rest.
@@ -471,12 +474,14 @@ int mgb_launch_cg_pupdate(const MeshDev *m, const Inst *insts, const int *list, 
 
 // The iterations of the listed instances after mgb_launch_cg_setup, to the end, in one cooperative launch.  Returns
 // -1 without launching where the batch is too large for it to pay (see kSolveNodes) or the device cannot hold it.
-int mgb_launch_cg_solve(const MeshDev *m, const Inst *insts, const int *list, int nlist, cudaStream_t s) {
+int mgb_launch_cg_solve(const MeshDev *m, const Inst *insts, const int *list, int nlist, int at_work, int parts,
+                        cudaStream_t s) {
   if (nlist <= 0) return 0;
-  if ((long long)m->nn * nlist > kSolveNodes) return -1;
-  const int sms = coop_sms();
-  if (!sms) return -1;
+  if ((long long)m->nn * nlist * (at_work > 1 ? at_work : 1) > kSolveNodes) return -1;
+  const int all = coop_sms();
+  if (!all) return -1;
   const int units = (int)cdiv(m->nn, 32);
+  const int sms = all > parts ? all / parts : 1;
   // groups of blocks that each take one instance after the other: the number that the iterations' times ask for
   // (kUnitUs per unit of a block, at least kChainUs, and kPhasesUs of barriers and scalars)
   int groups = 1, G = sms;

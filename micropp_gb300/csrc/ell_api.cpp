@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "at_work.hpp"
 #include "device.cuh"
 #include "ell_api.h"
 #include "launch.h"
@@ -54,7 +55,9 @@ int run_dpcg(const MeshDev &m, Inst *d_inst, int *d_list, unsigned int *d_count,
   chk((cudaError_t)mgb_launch_cg_setup(&m, d_inst, d_list, 1, s), "cg setup");
   const int chunk = (m.nn > 200000) ? 8 : 32;
   unsigned int count = 0;
-  const int one = mgb_launch_cg_solve(&m, d_inst, d_list, 1, s);
+  // all SMs: the allocations of calls that overlap wait for the device, so their solves run one after the other anyway (4
+  // of 30^3 nodes 23.5 ms, and 29 with half of the SMs each)
+  const int one = mgb_launch_cg_solve(&m, d_inst, d_list, 1, AtWork::count(), 1, s);
   if (one > 0) chk((cudaError_t)one, "cg solve");
   for (int done = 0; one < 0 && done <= max_its; done += chunk) {
     for (int it = 0; it < chunk; ++it) {
@@ -81,6 +84,7 @@ using namespace mgb;
 extern "C" int micropp3_ell_solve_cgpd(const int nodes[3], const double *vals, const double *b, double *x,
                                        double rel_tol, double abs_tol, int max_its, int *its, void *stream) {
   if (!nodes || !vals || !b || !x || nodes[0] < 2 || nodes[1] < 2 || nodes[2] < 2 || max_its < 0) return -1;
+  const AtWork at_work;
   const MeshDev m = stencil_mesh(nodes);
   const size_t nd = (size_t)m.nn * 3;
   const int nblocks = (int)((nd + kNodeBlock - 1) / kNodeBlock) + 8;

@@ -19,6 +19,7 @@
 #include <sstream>
 #include <stdexcept>
 
+#include "at_work.hpp"
 #include "cuda_util.hpp"
 #include "launch.h"
 #include "microstructure.hpp"
@@ -249,7 +250,10 @@ Engine::Engine(const micropp3_config &cfg) {
   }
 
   std::memset(ctan_lin_, 0, sizeof(ctan_lin_));
-  if (calc_ctan_lin_ && n_fe > 0) calc_ctan_lin();
+  if (calc_ctan_lin_ && n_fe > 0) {
+    const AtWork at_work;
+    calc_ctan_lin();
+  }
   for (auto &g : gps_) {
     if (g.coupling == MICROPP3_MIX_RULE_CHAMIS)
       ctan_mix_rule_chamis(g.ctan);
@@ -922,7 +926,8 @@ void Engine::cg_solve(const std::vector<int> &slots) {
   const int chunk = (mesh_.nn > 200000) ? 8 : 32;
   int done_its = 0;
   if (!timing_on()) {  // the per-kernel timers need the iterations launched kernel by kernel
-    const int e = mgb_launch_cg_solve(&mesh_, d_insts_, d_list_, n, stream_);
+    const int e = mgb_launch_cg_solve(&mesh_, d_insts_, d_list_, n, AtWork::count(), AtWork::parts(),
+                                      stream_);
     if (e >= 0) {
       check_launch(e, "cg solve");
       launches_ += 1;
@@ -1823,6 +1828,7 @@ void Engine::homogenize() {
     }
   }
   if (!fe.empty()) {
+    const AtWork at_work;
     // Slots for as many points as memory allows (at most all of them).
     size_t free_b = 0, total_b = 0;
     check(cudaMemGetInfo(&free_b, &total_b), "mem info");

@@ -43,8 +43,10 @@ int mgb_launch_cg_pupdate(const mgb::MeshDev *m, const mgb::Inst *insts, const i
 
 // All iterations after mgb_launch_cg_setup in one cooperative launch, bit for bit those of the three launches
 // above; -1 (nothing launched) where that does not pay.  An instance whose out.stalled is set
-// afterwards was not solved, and its ticket is to be cleared.
-int mgb_launch_cg_solve(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, cudaStream_t s);
+// afterwards was not solved, and its ticket is to be cleared.  at_work: how many handles use the GPU (AtWork); 1 / parts of
+// the SMs are taken.  Neither changes a result.
+int mgb_launch_cg_solve(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, int at_work, int parts,
+                        cudaStream_t s);
 
 int mgb_launch_assembly32(const mgb::MeshDev *m, const mgb::Mats *mats, const int8_t *etype, const double *dsh,
                           const float *ke_phase, const mgb::Inst *insts, const int *list, int nlist, void *ring,

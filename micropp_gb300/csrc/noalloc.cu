@@ -24,6 +24,7 @@
 #include <cstdio>
 #include <stdexcept>
 
+#include "at_work.hpp"
 #include "device.cuh"
 #include "ell_api.h"
 #include "micropp_gb300.h"
@@ -83,6 +84,7 @@ extern "C" int micropp3_ell_solve_cgpd_noalloc(const int nodes[3], const double 
                  nn, MICROPP3_NOALLOC_MAX_NODES);
     return -3;
   }
+  const AtWork at_work;
   unsigned char *base = nullptr;
   cudaError_t e = scratch_address(&base);
   if (e != cudaSuccess) return (int)e;

@@ -14,6 +14,7 @@
 #include <cstring>
 #include <stdexcept>
 
+#include "at_work.hpp"
 #include "cuda_util.hpp"
 #include "engine.hpp"
 #include "launch.h"
@@ -124,6 +125,7 @@ struct PathScope {
 int Engine::path_forward(int nsteps, const double *strains, const double *params, int every, double *sigma) {
   if (nsteps <= 0 || !strains || !params || !sigma || every <= 0)
     throw std::invalid_argument("path: nsteps > 0, strains, params, sigma and checkpoint_every > 0 are required");
+  const AtWork at_work;
   path_free();
   PathState &P = path_;
   P.nsteps = nsteps;
@@ -242,6 +244,7 @@ int Engine::path_vjp(const double *gsigma, double *grad_params, double *grad_str
   PathState &P = path_;
   if (!P.ready) throw std::runtime_error("path_vjp: no path (call micropp3_path_forward first)");
   if (!gsigma || !grad_params) throw std::invalid_argument("path_vjp: gsigma and grad_params are required");
+  const AtWork at_work;
   const size_t nd = nndim(), nv = nvars();
   ensure_fp64_slot0();
   if (P.seg_u.empty())

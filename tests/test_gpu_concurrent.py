@@ -1,0 +1,77 @@
+"""Handles at work at the same time: each one-launch solve leaves SMs to the others.  The count of handles decides how many
+blocks a solve takes, never its result: every sum has an order that does not depend on them."""
+import ctypes
+import time
+
+import numpy as np
+import pytest
+
+from cases import gpu_config
+from micropp_gb300 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+MATS = {"elastic": (0, 1e7, 0.25, 0, 0, 0), "damage": (2, 1e7, 0.25, 0, 0, 1e5), "j2": (1, 1e7, 0.3, 1e5, 1e4, 0)}
+PLAIN = dict(nr_max_its=6, nr_max_tol=1e-5, calc_ctan_lin=0)
+
+
+def handles(specs, **form):
+    """(handle, strains) per (elements, points, law)."""
+    import micropp_gb300 as mg
+    out = []
+    for i, (n, ngp, law) in enumerate(specs):
+        kw = dict(ngp=ngp, mats=(MATS[law], (0, 1e8, 0.25, 0, 0, 0), (0, 1e7, 0.25, 0, 0, 0)), lin_stress=0,
+                  micro_type=1, geo=(0.2, 0, 0, 0), **form)
+        kw.setdefault("coupling", [1] * ngp)
+        out.append((mg.Micropp(gpu_config(n, **kw)), wl.random_targets(ngp, 40 + i, 2.5e-2 if law == "damage" else 5e-3)))
+    return out
+
+
+def homogenize(hs):
+    """All handles at once; results and seconds."""
+    import micropp_gb300 as mg
+    lib = mg.load()
+    for h, strains in hs:
+        for gp, e in enumerate(strains):
+            h.set_strain(gp, e)
+    arr = (ctypes.POINTER(mg.Handle) * len(hs))(*[ctypes.pointer(h.h) for h, _ in hs])
+    t = time.perf_counter()
+    lib.micropp3_homogenize_many(arr, len(hs))
+    t = time.perf_counter() - t
+    assert not lib.micropp3_last_error()
+    return [(h.get_stress(gp), h.get_ctan(gp), h.u(gp, 1), h.newton(gp), h.get_cost(gp), h.status(gp))
+            for h, s in hs for gp in range(len(s))], t
+
+
+def same(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a[:3], b[:3])) and a[3:] == b[3:]
+
+
+def at_once_over_in_turn(hs, repeats=3):
+    """Seconds of all handles at once over those of one after the other (least of `repeats`)."""
+    for h in hs:
+        homogenize([h])
+    return min(homogenize(hs)[1] for _ in range(repeats)) / sum(min(homogenize([h])[1] for _ in range(repeats)) for h in hs)
+
+
+# fewer units than a share has SMs, shares with several units per block and per group of warps, batches, and batches that
+# are launched kernel by kernel only when there are so many of them
+@pytest.mark.parametrize("specs", [
+    [(6, 1, "j2"), ((7, 4, 9), 3, "damage"), (2, 5, "damage")], [(20, 1, "j2")] * 5, [(12, 8, "damage")] * 10,
+    [(30, 1, "damage"), (25, 2, "j2"), (30, 2, "damage"), (26, 1, "damage")]])
+def test_plain_handles_at_once_are_bitwise_the_lone_ones(gpu_lib, specs):
+    hs = handles(specs, **PLAIN)
+    lone = [r for h in hs for r in homogenize([h])[0]]
+    for _ in range(2):
+        assert all(same(a, b) for a, b in zip(lone, homogenize(hs)[0]))
+    for h, _ in hs:
+        h.close()
+
+
+def test_plain_handles_overlap(gpu_lib):
+    """16 J2 points of 20^3, a handle each: a solve that takes every SM makes the others wait, and all of them at once then
+    take as long as one after the other."""
+    hs = handles([(20, 1, "j2")] * 16, **PLAIN)
+    assert at_once_over_in_turn(hs) < 0.75
+    for h, _ in hs:
+        h.close()
