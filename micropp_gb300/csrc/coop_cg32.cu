@@ -15,6 +15,10 @@
 // vectors of the 1-RHS solve are component-major here, as those of the 6-RHS solve (du32 and kinv32 alone stay
 // node-interleaved): 32 nodes are one 128-byte access.
 //
+// A sum over an instance is formed over V parts, the blocks of a solve that has all SMs.  With fewer blocks (other handles
+// are at work) a block has several parts and forms the sum of each as a block of its own would: the result does not depend
+// on what else runs.  That is a kernel of its own (SHARED): in one body the solve with a part per block was 1.5-3% slower.
+//
 // Arithmetic: every FP32 sum -- the products of a row, a thread's part of a dot product, the 32 lanes of a warp --
 // is formed as in the launched kernels (mixed_kernels.cu, mg_kernels.cu), in their order; the FP64 sums above a warp
 // are not, which changes an FP32 scalar once in 1e8 or so.  The outputs of the two forms are the same but for that.
@@ -36,12 +40,21 @@ constexpr int kHeldFloats = kGroups * kUnitFloats;
 // Blocks per instance from which one of them keeps to the tail: below, a block more for the other levels is worth more.
 constexpr int kTailBlocks = 8;
 
+// Parts of the sums that a block sets down between two __syncthreads.
+constexpr int kPass = 8;
+
 // Batches solved by one cooperative launch: at most kCoopNodes nodes in all and kTailBlocks blocks for each instance,
 // or with the V-cycle half as many blocks and kCoopNodesFew nodes.  One homogenization (stress and ctan, damage,
 // multigrid), launched and here, ms: 60^3 x 1 20.3 and 14.5, x 4 47.3 and 44.5; 40^3 x 8 33.1 and 28.3, x 16 53.7 and
 // 55.4; 30^3 x 32 46.9 and 49.2; 20^3 x 32 21.1 and 18.4, x 100 50.9 and 56.4; 10^3 x 32 9.7 and 5.9, x 200 25.2 and
 // 26.6; Jacobi 20^3 x 32 24.2 and 25.2, 40^3 x 4 41.6 and 40.0.
-constexpr long long kCoopNodes = 950000, kCoopNodesFew = 300000;
+//
+// Handles homogenized together (launched, one launch with a share of the SMs, one launch with all of them; ms): multigrid,
+// a point of 30^3 each, x 4 19.7, 11.6, 15.1, x 16 48.3, 33.6, 53.2; 40^3 x 16 82.3, 65.7, 82.7.  Jacobi 30^3 x 4 24.5,
+// 18.6, 24.0, x 8 32.6, 31.8, 45.6, 40^3 x 3 36.4, 35.3, 38.1; above kCoopBeside nodes in all its solves are launched: 40^3 x
+// 4 40.0, 45.1, 50.3, 30^3 x 16 54.8, 57.4, 87.2, 60^3 x 4 163, 200, 224 -- without the V-cycle's latencies the products
+// bound an iteration, and those of six right-hand sides are slower here.
+constexpr long long kCoopNodes = 950000, kCoopNodesFew = 300000, kCoopBeside = 250000;
 
 // Nodes per warp of the launched kernels' dot products, in units of 32: blocks own whole multiples.
 __host__ __device__ constexpr int own_units(int nr) { return nr == 1 ? 4 : 2; }
@@ -81,13 +94,16 @@ struct Ctx {
   unsigned int *ctr;
   uint64_t policy;  // L2 eviction priority of the matrix values
   double min_err, rel_err;
-  double warp[2][kWarps], tot[12], rz[6], pn0[6];
+  double tot[12], rz[6], pn0[6];
   float alpha[6], beta[6];
   int rdone[6], done, ok, bad;
   int held[kGroups];  // the unit (level << 24 | unit) whose values each group of 3 warps holds
   int me, workers;    // this block among those that work on the levels before the tail (me = -1: the tail's block)
-  int u0, u1;         // its level-0 units
-  int G, rank, pairs;
+  int u0, u1;         // its level-0 units, those of its parts v0 .. v1 - 1
+  int V, v0, v1;
+  int idle;           // parts without level-0 units: 1 where a solve with all SMs has a block for the tail
+  int pairs;
+  double warp[2][kPass][kWarps];
 };
 constexpr int kCtxBytes = (sizeof(Ctx) + 127) / 128 * 128;
 
@@ -522,16 +538,31 @@ __device__ __noinline__ void fill_tail() {
   __syncthreads();
 }
 
-// This warp's part (lane 0) of x.y over the block's level-0 nodes: `per` nodes per thread, as the launched kernel whose
-// sum it is.
+// First level-0 unit of part v (v = V: the end): runs of whole own_units.
 template <int NR>
-__device__ __noinline__ double dot0(const float *x, const float *y, int per) {
+__device__ __forceinline__ int first_unit(const Ctx &c, int v) {
+  const int runs = (c.lv.g[0].units + own_units(NR) - 1) / own_units(NR);
+  if (v <= c.idle) return 0;
+  return min(runs * (v - c.idle) / (c.V - c.idle) * own_units(NR), c.lv.g[0].units);
+}
+
+// Level-0 units u0 .. u1 - 1 of the block's part v
+template <int NR, bool SHARED>
+__device__ __forceinline__ int2 part_units(const Ctx &c, int v) {
+  return SHARED ? make_int2(first_unit<NR>(c, v), first_unit<NR>(c, v + 1)) : make_int2(c.u0, c.u1);
+}
+
+// Warp `wid`'s share (lane 0) of x.y over the level-0 nodes of part v: `per` nodes per thread, as the launched kernel whose
+// sum it is.
+template <int NR, bool SHARED>
+__device__ __noinline__ double dot0(const float *x, const float *y, int per, int v, int wid) {
   const Ctx &c = ctx();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = wid % NR, nn = c.lv.g[0].nn;
+  const int lane = threadIdx.x & 31, q = wid % NR, nn = c.lv.g[0].nn;
+  const int2 u = part_units<NR, SHARED>(c, v);
   const size_t np = c.lv.g[0].np;
   double acc = 0.0;
-  for (int w = wid / NR; w * per < c.u1 - c.u0; w += kWarps / NR) {
-    const int n = (c.u0 + w * per) * 32 + lane * per;
+  for (int w = wid / NR; w * per < u.y - u.x; w += kWarps / NR) {
+    const int n = (u.x + w * per) * 32 + lane * per;
     float xv[4][3], yv[4][3], s = 0.f;
 #pragma unroll
     for (int p = 0; p < 4; ++p)
@@ -552,12 +583,13 @@ __device__ __noinline__ double dot0(const float *x, const float *y, int per) {
   return acc;
 }
 
-// D += alpha P; R -= alpha AP; Z = D^-1 R (the V-cycle's start) or kinv R; this warp's part of the stop test's norm
-// and, with the Jacobi preconditioner, of r.z.  Rows are dealt to the warps as the launched updates deal them.
+// D += alpha P; R -= alpha AP; Z = D^-1 R (the V-cycle's start) or kinv R; for warp `wid` of part v, with its share of the
+// stop test's norm and, with the Jacobi preconditioner, of r.z.  Rows are dealt to the parts and their warps as the
+// launched updates deal them.
 template <int NR, bool MG>
-__device__ __noinline__ double2 update() {
+__device__ __noinline__ double2 update(int v, int wid) {
   const Ctx &c = ctx();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nn = c.lv.g[0].nn;
+  const int lane = threadIdx.x & 31, nn = c.lv.g[0].nn;
   const size_t np = c.lv.g[0].np;
   float *R = c.R, *Z = c.Z, *D = c.D;
   const float *P = c.P, *AP = c.AP, *kinv = c.kinv, *ks = c.ks;
@@ -565,7 +597,7 @@ __device__ __noinline__ double2 update() {
   if (NR == 1) {
     const int nrow = nn * 3, ublocks = (nrow + 1023) / 1024, ustride = ublocks * 256;
     const float al = c.alpha[0];
-    for (int w = wid * c.G + c.rank; w < ublocks * 8; w += c.G * kWarps) {
+    for (int w = wid * c.V + v; w < ublocks * 8; w += c.V * kWarps) {
       float zz = 0.f, rz = 0.f, pv[4], av[4], rv[4], dv[4], kv[4], sv[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -595,7 +627,7 @@ __device__ __noinline__ double2 update() {
   } else if (!c.rdone[wid % NR]) {
     const int q = wid % NR, wchunks = (nn + 1023) / 1024 * 8;
     const float al = c.alpha[q];
-    for (int w = (wid / NR) * c.G + c.rank; w < wchunks; w += c.G * (kWarps / NR)) {
+    for (int w = (wid / NR) * c.V + v; w < wchunks; w += c.V * (kWarps / NR)) {
       const int n0 = (w >> 3) * 1024 + (w & 7) * 32 + lane;
       float zz = 0.f, rz = 0.f;
 #pragma unroll
@@ -665,15 +697,17 @@ __device__ __noinline__ void direction(bool start) {
   }
 }
 
-// Start of a 1-RHS solve: R = b, D = 0, the inverse diagonal, Z (P) and this warp's part of ||kinv r||^2 and r.z
-template <bool MG>
-__device__ __noinline__ double2 setup1() {
+// Start of a 1-RHS solve: R = b, D = 0, the inverse diagonal, Z (P) and the share of warp `wid` of part v of ||kinv r||^2
+// and r.z
+template <bool MG, bool SHARED>
+__device__ __noinline__ double2 setup1(int v, int wid) {
   const Ctx &c = ctx();
   const Grid &g = c.lv.g[0];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int2 units = part_units<1, SHARED>(c, v);
+  const int lane = threadIdx.x & 31;
   const size_t np = g.np;
   double azz = 0.0, arz = 0.0;
-  for (int u = c.u0 + wid; u < c.u1; u += kWarps) {
+  for (int u = units.x + wid; u < units.y; u += kWarps) {
     const int n = u * 32 + lane;
     float zz = 0.f, rz = 0.f;
     if (n < g.nn) {
@@ -698,19 +732,19 @@ __device__ __noinline__ double2 setup1() {
   return make_double2(azz, arz);
 }
 
-template <int NR, bool MG>
+template <int NR, bool MG, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_coop_cg32(Levels lv, const Inst *insts, const int *list, int G, const double *rel_tols, double abs_tol,
-                int max_its_arg, int pairs, float keep) {
+    k_coop_cg32(Levels lv, const Inst *insts, const int *list, int G, int V, int idle, const double *rel_tols,
+                double abs_tol, int max_its_arg, int pairs, float keep) {
   Ctx &c = ctx();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int a = blockIdx.x / G, rank = blockIdx.x - a * G;
   const bool tail = MG && lv.tail < lv.n;
   if (tid == 0) {
-    // rank 0 keeps to the tail; the units of the other levels go to the workers, in runs of whole own_units on level 0
+    // rank 0 keeps to the tail; the units of the other levels go to the workers, on level 0 by the parts of the sums
     c.lv = lv;
-    c.G = G;
-    c.rank = rank;
+    c.V = V;
+    c.idle = idle;
     c.pairs = pairs;
     uint64_t policy = 0;
     if (keep < 1.f)
@@ -718,9 +752,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     c.policy = policy;
     c.workers = tail ? G - 1 : G;
     c.me = tail ? rank - 1 : rank;
-    const int runs = (lv.g[0].units + own_units(NR) - 1) / own_units(NR);
-    c.u0 = c.me < 0 ? 0 : runs * c.me / c.workers * own_units(NR);
-    c.u1 = c.me < 0 ? 0 : min(runs * (c.me + 1) / c.workers * own_units(NR), lv.g[0].units);
+    const int first = tail ? 1 : 0;  // parts of rank 0 alone
+    c.v0 = c.me < 0 ? 0 : first + (V - first) * c.me / c.workers;
+    c.v1 = c.me < 0 ? 1 : first + (V - first) * (c.me + 1) / c.workers;
+    c.u0 = first_unit<NR>(c, c.v0);
+    c.u1 = first_unit<NR>(c, c.v1);
   }
   const Inst &I = insts[list[a]];
   Cg6State *c6s = I.cg6;
@@ -763,28 +799,44 @@ __global__ void __launch_bounds__(kThreads, 1)
     ok = group_barrier(c.ctr, target, &c.ok);
     return ok;
   };
-  // Sums over the instance of the lanes 0' values v0 and v1 (those of warp w belong to right-hand side w % NR): a
-  // barrier, after which c.tot[kind * NR + q] holds them.  Two buffers of partials in turn: a block may write the
-  // next ones while another still reads these.
-  auto reduce = [&](double v0, double v1, int kinds) {
-    if (lane == 0) {
-      c.warp[0][wid] = v0;
-      c.warp[1][wid] = v1;
-    }
-    __syncthreads();
-    double *part = c.red + (size_t)turn * 2 * NR * G;
+  // Sums over the instance of what share(v, w) returns in lane 0 for warp w of the block's part v (the values of warp w
+  // belong to right-hand side w % NR): a barrier, after which c.tot[kind * NR + q] holds them.  Two buffers of partials in
+  // turn: a block may write the next ones while another still reads these.
+  auto reduce = [&](auto share, int kinds) {
+    double *part = c.red + (size_t)turn * 2 * NR * V;
     turn ^= 1;
-    if (tid < kinds * NR) {
-      const int kind = tid / NR, q = tid - kind * NR;
+    // sum k of part p0 + i
+    auto set_down = [&](int p0, int i, int k) {
+      const int kind = k / NR, q = k - kind * NR;
       double v = 0.0;
 #pragma unroll
-      for (int w = 0; w < kWarps / NR; ++w) v += c.warp[kind][w * NR + q];
-      part[(size_t)tid * G + rank] = v;
+      for (int w = 0; w < kWarps / NR; ++w) v += c.warp[kind][i][w * NR + q];
+      part[(size_t)k * V + p0 + i] = v;
+    };
+    auto keep_share = [&](double2 r, int i, int w) {
+      if (lane == 0) {
+        c.warp[0][i][w] = r.x;
+        c.warp[1][i][w] = r.y;
+      }
+    };
+    if constexpr (SHARED) {
+      for (int p0 = c.v0; p0 < c.v1; p0 += kPass) {
+        const int n = min(kPass, c.v1 - p0);
+        // a part has fewer units than warps: the warps take turns at the first ones
+        for (int i = 0, w = wid; i < n; ++i, w = w < kWarps - 6 ? w + 6 : w + 6 - kWarps) keep_share(share(p0 + i, w), i, w);
+        __syncthreads();
+        for (int e = tid; e < kinds * NR * n; e += kThreads) set_down(p0, e / (kinds * NR), e % (kinds * NR));
+        if (p0 + kPass < c.v1) __syncthreads();
+      }
+    } else {
+      keep_share(share(rank, wid), 0, wid);
+      __syncthreads();
+      if (tid < kinds * NR) set_down(rank, 0, tid);
     }
     if (!barrier()) return false;
     if (wid < kinds * NR) {
       double v = 0.0;
-      for (int b = lane; b < G; b += 32) v += __ldcg(part + (size_t)wid * G + b);
+      for (int b = lane; b < V; b += 32) v += __ldcg(part + (size_t)wid * V + b);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       if (lane == 0) c.tot[wid] = v;
@@ -822,7 +874,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     apply<NR>(kPost, 0, 0, 0);
     __syncthreads();
-    return reduce(dot0<NR>(c.R, c.Z, NR == 1 ? 1 : 2), 0.0, 1);
+    return reduce([&](int v, int w) { return make_double2(dot0<NR, SHARED>(c.R, c.Z, NR == 1 ? 1 : 2, v, w), 0.0); }, 1);
   };
   auto all_done = [&]() {
     __syncthreads();
@@ -851,8 +903,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   double pnorm = 0.0;
   fill_tail<NR>();
   if (NR == 1) {
-    const double2 v = setup1<MG>();
-    run = reduce(v.x, v.y, 2);
+    run = reduce([&](int v, int w) { return setup1<MG, SHARED>(v, w); }, 2);
     if (run) {
       const double zz = c.tot[0], rz = c.tot[1], pn = sqrt(zz);
       pnorm = pn;
@@ -878,11 +929,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   while (run) {
     apply<NR>(kProduct, 0, 0, 0);
     __syncthreads();
-    if (!reduce(dot0<NR>(c.P, c.AP, own_units(NR)), 0.0, 1)) break;
+    if (!reduce([&](int v, int w) { return make_double2(dot0<NR, SHARED>(c.P, c.AP, own_units(NR), v, w), 0.0); }, 1)) break;
     if (tid < NR) c.alpha[tid] = c.rdone[tid] ? 0.f : (float)(c.rz[tid] / c.tot[tid]);
     __syncthreads();
-    const double2 v = update<NR, MG>();
-    if (!reduce(v.x, v.y, MG ? 1 : 2)) break;
+    if (!reduce([&](int v, int w) { return update<NR, MG>(v, w); }, MG ? 1 : 2)) break;
     its += 1;
     if (tid < NR && !c.rdone[tid]) {
       const double tot = c.tot[tid], pn = sqrt(tot);
@@ -952,14 +1002,14 @@ float keep_fraction(double bytes) {
 }
 
 template <int NR, bool MG>
-int launch(const Levels &lv, const Inst *insts, const int *list, int nlist, int G, const double *rel_tols,
-           double abs_tol, int max_its, int pairs, float keep, cudaStream_t s) {
+int launch(const Levels &lv, const Inst *insts, const int *list, int nlist, int G, int V, int idle,
+           const double *rel_tols, double abs_tol, int max_its, int pairs, float keep, cudaStream_t s) {
   Levels l = lv;
   const size_t smem = kCtxBytes + kHeldFloats * sizeof(float);
-  const void *f = (const void *)k_coop_cg32<NR, MG>;
+  const void *f = G < V ? (const void *)k_coop_cg32<NR, MG, true> : (const void *)k_coop_cg32<NR, MG, false>;
   cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  void *args[] = {&l, &insts, &list, &G, &rel_tols, &abs_tol, &max_its, &pairs, &keep};
+  void *args[] = {&l, &insts, &list, &G, &V, &idle, &rel_tols, &abs_tol, &max_its, &pairs, &keep};
   e = cudaLaunchCooperativeKernel(f, dim3(nlist * G), dim3(kThreads), args, smem, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
@@ -975,24 +1025,26 @@ using namespace mgb;
 
 extern "C" {
 
-int mgb_coop_cg32_pays(const MeshDev *m, int nlist, int mg) {
+int mgb_coop_cg32_pays(const MeshDev *m, int nlist, int mg, long long beside) {
   const long long nodes = (long long)m->nn * nlist;
   if (nlist <= 0 || nodes > kCoopNodes) return 0;
+  if (!mg && beside > kCoopBeside) return 0;
   const int blocks = coop_sms() / nlist;
   return blocks >= kTailBlocks || (mg && blocks >= kTailBlocks / 2 && nodes <= kCoopNodesFew);
 }
 
 int mgb_launch_coop_cg32(const MeshDev *levels, int nlevels, const Inst *insts, const int *list, int nlist, int nr,
-                         const double *rel_tols, double abs_tol, int max_its, int pairs, cudaStream_t s) {
+                         const double *rel_tols, double abs_tol, int max_its, int pairs, int parts, cudaStream_t s) {
   if (nlist <= 0) return 0;
   if (nlevels < 1 || nlevels > kMgMaxLevels || (nr != 1 && nr != 6)) return (int)cudaErrorInvalidValue;
-  int G = coop_sms() / nlist, tail = 0;  // blocks per instance, one per SM
-  if (G < 1) return -1;
+  const int sms = coop_sms();
+  int V = sms / nlist, tail = 0;  // blocks per instance, one per SM
+  if (V < 1) return -1;
   Levels lv{};
   lv.n = lv.tail = nlevels;
   for (int l = 0; l < nlevels; ++l) lv.g[l] = grid_of(levels[l]);
   const int runs = (lv.g[0].units + own_units(nr) - 1) / own_units(nr);
-  if (G >= kTailBlocks)
+  if (V >= kTailBlocks)
     for (int l = nlevels - 1; l >= 1; --l) {
       const int more = tail_floats(lv.g[l], nr);
       if (tail + more > kHeldFloats || lv.g[l].inner == 0) break;
@@ -1002,12 +1054,17 @@ int mgb_launch_coop_cg32(const MeshDev *levels, int nlevels, const Inst *insts, 
   // no more workers than have a run (1 RHS) or a unit for each group of warps (6 RHS): the rest of the SMs is better
   // left to the solves of other handles
   const int per = nr == 1 ? 1 : kGroups / own_units(6), most = (runs + per - 1) / per + (lv.tail < nlevels ? 1 : 0);
-  if (G > most) G = most;
+  if (V > most) V = most;
+  const int idle = lv.tail < nlevels ? 1 : 0;
+  // with a share of the SMs: fewer blocks than parts of the sums
+  int G = sms / (nlist * parts);
+  G = G < 1 ? 1 : G < V ? G : V;
+  if (G < V && G < kTailBlocks) lv.tail = nlevels;
   const bool mg = nlevels > 1;
   const float keep = keep_fraction((double)kEllPerNode * sizeof(float) * levels[0].np * nlist);
 #define MGB_COOP(NR)                                                                                                  \
-  (mg ? launch<NR, true>(lv, insts, list, nlist, G, rel_tols, abs_tol, max_its, pairs, keep, s)                     \
-      : launch<NR, false>(lv, insts, list, nlist, G, rel_tols, abs_tol, max_its, pairs, keep, s))
+  (mg ? launch<NR, true>(lv, insts, list, nlist, G, V, idle, rel_tols, abs_tol, max_its, pairs, keep, s)            \
+      : launch<NR, false>(lv, insts, list, nlist, G, V, idle, rel_tols, abs_tol, max_its, pairs, keep, s))
   return nr == 1 ? MGB_COOP(1) : MGB_COOP(6);
 #undef MGB_COOP
 }

@@ -972,7 +972,7 @@ void Engine::cg_init(const std::vector<double> &rel_tols, int max_its) {
 // Whether an FP32 solve of n listed instances runs in one cooperative launch: batches small enough, unless
 // per-kernel timers want the iterations launched kernel by kernel or the V-cycle reads the FP16 operator.
 bool Engine::coop32(int n, bool use_mg) const {
-  return !timing_on() && !(mg_ && use_mg && mg_half_) && mgb_coop_cg32_pays(&mesh_, n, mg_ && use_mg);
+  return !timing_on() && !(mg_ && use_mg && mg_half_) && mgb_coop_cg32_pays(&mesh_, n, mg_ && use_mg, beside_);
 }
 
 // That launch for the n instances in d_list_ (nr = 1: with the tolerances in d_eta_; nr = 6: after the tangent
@@ -981,7 +981,7 @@ bool Engine::coop_solve32(int n, int nr, bool use_mg) {
   const bool mg = mg_ && use_mg;
   const int e = mgb_launch_coop_cg32(mg ? mg_mesh_.data() : &mesh_, mg ? (int)mg_mesh_.size() : 1, d_insts_, d_list_, n,
                                      nr, d_eta_, cg_abs_tol_, mg ? std::min(cg_max_its_, kMgMaxIts) : cg_max_its_,
-                                     kMgCoarsePairs, stream_);
+                                     kMgCoarsePairs, AtWork::parts(), stream_);
   if (e < 0) return false;
   check_launch(e, "cg solve (FP32)");
   launches_ += 1;

@@ -147,6 +147,9 @@ class Engine {
   void set_kernel_timing(bool on);
   bool kernel_stats(const std::string &family, long *launches, double *ms, double *bytes);
   long total_cg_its() const { return total_cg_its_; }
+  // Nodes of all points of the handle, and of those that micropp3_homogenize_many has at work with it (0: none).
+  long long point_nodes() const { return (long long)mesh_.nn * ngp_; }
+  void set_beside(long long nodes) { beside_ = nodes; }
   long kernel_launches() const { return launches_; }
   int mpi_rank() const { return mpi_rank_; }
 
@@ -264,6 +267,7 @@ class Engine {
   unsigned int *d_count_ = nullptr, *h_count_ = nullptr;
   double last_ms_ = 0.0;
   long total_cg_its_ = 0;
+  long long beside_ = 0;
   long launches_ = 0;  // kernels of this library launched by the handle
   KernelTimer t_spmv_, t_update_, t_asm_, t_res_, t_spmv6_, t_upd6_;
   KernelTimer t_rap_;  // multigrid operators after an assembly: smoother diagonals and Galerkin products

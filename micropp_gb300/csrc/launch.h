@@ -89,11 +89,12 @@ int mgb_launch_t6_residual(const mgb::MeshDev *m, const mgb::Inst *insts, const 
 // All iterations of an FP32 CG solve of nr = 1 or 6 right-hand sides in one cooperative launch (coop_cg32.cu); levels:
 // the grids of the V-cycle, finest first (one level: Jacobi).  nr = 1: from b, with rel_tols[a] for the a-th listed
 // instance; nr = 6: from the state mgb_launch_t6_residual leaves.  An instance whose out.stalled is set afterwards
-// was not solved, and its ticket is to be cleared.  -1: not available, nothing launched.  _pays: whether it is the faster
-// form for a batch.
-int mgb_coop_cg32_pays(const mgb::MeshDev *m, int nlist, int mg);
+// was not solved, and its ticket is to be cleared.  1 / parts of the SMs are taken, which changes no result.  -1: not
+// available, nothing launched.  _pays: whether it is the faster form for a batch;
+// beside: nodes of all handles of one micropp3_homogenize_many call (0: none).
+int mgb_coop_cg32_pays(const mgb::MeshDev *m, int nlist, int mg, long long beside);
 int mgb_launch_coop_cg32(const mgb::MeshDev *levels, int nlevels, const mgb::Inst *insts, const int *list, int nlist,
-                         int nr, const double *rel_tols, double abs_tol, int max_its, int pairs, cudaStream_t s);
+                         int nr, const double *rel_tols, double abs_tol, int max_its, int pairs, int parts, cudaStream_t s);
 int mgb_launch_cg6_spmv(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, int block,
                         cudaStream_t s);
 int mgb_launch_cg6_update(const mgb::MeshDev *m, const mgb::Inst *insts, const int *list, int nlist, int mg,

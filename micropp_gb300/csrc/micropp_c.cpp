@@ -249,10 +249,16 @@ void micropp3_homogenize_many(struct micropp3 *const *handles, int n) {
     }
   };
   const int nthreads = std::min(n, 16);
+  // The form of a solve goes by what is homogenized with it: known from the call, so that its results do not depend on
+  // which handle is where.
+  long long nodes = 0;
+  for (const Engine *e : engines) nodes += e->point_nodes();
+  for (Engine *e : engines) e->set_beside(n > 1 ? nodes * nthreads / n : 0);
   std::vector<std::thread> pool;
   for (int t = 1; t < nthreads; ++t) pool.emplace_back(work);
   work();
   for (auto &t : pool) t.join();
+  for (Engine *e : engines) e->set_beside(0);
   for (int i = 0; i < n; ++i)
     if (!errors[i].empty()) fail("micropp3_homogenize_many", ("handle " + std::to_string(i) + ": " + errors[i]).c_str());
 }

@@ -1,5 +1,6 @@
 """Handles at work at the same time: each one-launch solve leaves SMs to the others.  The count of handles decides how many
-blocks a solve takes, never its result: every sum has an order that does not depend on them."""
+blocks a solve takes, never its result: every sum has an order that does not depend on them.  (Jacobi solves of many large
+handles in one call are launched kernel by kernel, which rounds the FP64 sums in another order; the sizes here are below.)"""
 import ctypes
 import time
 
@@ -73,5 +74,32 @@ def test_plain_handles_overlap(gpu_lib):
     take as long as one after the other."""
     hs = handles([(20, 1, "j2")] * 16, **PLAIN)
     assert at_once_over_in_turn(hs) < 0.75
+    for h, _ in hs:
+        h.close()
+
+
+# FP32 solves with shares of several parts of the sums per block: with and without a block for the coarsest levels, batches
+# whose instances have a block each, one and six right-hand sides, and both preconditioners
+@pytest.mark.parametrize("precond", [0, 1], ids=["jacobi", "multigrid"])
+@pytest.mark.parametrize("specs", [
+    [(5, 1, "damage"), ((7, 5, 9), 3, "j2"), (8, 19, "elastic")], [(25, 1, "damage")] * 9, [(16, 8, "damage")] * 5,
+    [((13, 17, 23), 2, "j2"), (20, 1, "damage"), (40, 1, "damage"), (12, 16, "damage")]])
+def test_fast_handles_at_once_are_bitwise_the_lone_ones(gpu_lib, specs, precond):
+    import micropp_gb300 as mg
+    form = dict(wl.FAST_FORM, precond=precond, calc_ctan_lin=0)
+    hs = [handles([s], **form, coupling=[mg.FE_FULL] * s[1])[0] for s in specs]
+    hs = [(h, s * (1 + 0.1 * i)) for i, (h, s) in enumerate(hs)]
+    lone = [r for h in hs for r in homogenize([h])[0]]
+    for _ in range(2):
+        assert all(same(a, b) for a, b in zip(lone, homogenize(hs)[0]))
+    for h, _ in hs:
+        h.close()
+
+
+def test_fast_handles_overlap(gpu_lib):
+    """13 damage points of 25^3 with the Jacobi preconditioner, a handle each."""
+    import micropp_gb300 as mg
+    hs = handles([(25, 1, "damage")] * 13, **dict(wl.FAST_FORM, precond=0, calc_ctan_lin=0), coupling=[mg.FE_FULL])
+    assert at_once_over_in_turn(hs) < 0.7
     for h, _ in hs:
         h.close()
