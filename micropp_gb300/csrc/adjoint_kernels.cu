@@ -393,28 +393,49 @@ __global__ void __launch_bounds__(kNodeBlock) k_bicg_r(MeshDev m, AdjDev A, unsi
 // every phase.  A 12^3 J2 path of 4 steps, forward and reverse: 503 ms launched, 171 ms so.
 constexpr int kBicgUnit = 288;  // threads per unit
 constexpr int kBicgGroups = 3;  // units a block works on at a time, at most
+// A sum over the rows is formed over V parts, the blocks of a solve that has all SMs; with half of them (other handles are
+// at work) a block has up to kBicgParts parts, and the result is the same.  Damage paths of one step, a handle and a thread
+// each, on all SMs each, on halves, and launched, ms: 4 of 20^3 95.5, 87.5, 90.8, 16 of 16^3 257, 233, 188, 4 of 30^3 274,
+// 261, 262, 8 of 30^3 552, 523, 450; quarters of the SMs are slower again (16 of 20^3 366, halves 345).
+constexpr int kBicgShare = 2, kBicgParts = kBicgShare + 1;
 // Largest RVE (nodes) solved in one launch: the largest it was measured at.  The launched iteration is five kernels and
 // re-reads the vectors between them; a load step and its reverse pass (damage, edges of 6, 12, 20, 30, 45, 60, 75, 90)
 // take 21.6, 38.6, 61.9, 99, 335, 717, 1792, 2864 ms launched and 9.1, 14.3, 26.6, 74, 230, 568, 1408, 2673 in one
 // launch: the gain shrinks to 7% where the vectors outgrow L2.
 constexpr int kBicgNodes = 800000;
 
-template <bool Transpose>
-__global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDev m, AdjDev A, int units) {
+//
+// Shared: blocks with several parts.  A kernel of its own, since loops over the parts cost a solve with one each 5%.
+template <bool Transpose, bool Shared>
+__global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1)
+    k_bicg_solve(MeshDev m, AdjDev A, int units, int V, int groups_arg) {
   __shared__ double part_rows[2][kBicgGroups][9][32];
-  __shared__ double s_warp[2][kBicgUnit * kBicgGroups / 32];
+  __shared__ double s_warp[2][Shared ? kBicgParts : 1][9 * kBicgGroups];
   __shared__ double s_tot[2], s_alpha, s_beta, s_omega, s_rho;
   __shared__ int s_done, s_ok;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, G = gridDim.x, rank = blockIdx.x;
-  const int ug = tid / kBicgUnit, t = tid - ug * kBicgUnit, groups = blockDim.x / kBicgUnit, nwarps = blockDim.x >> 5;
+  const int ug = tid / kBicgUnit, t = tid - ug * kBicgUnit;
   const int fi = (t >> 5) % 3, dz = (t >> 5) / 3;
-  const int u0 = (int)((long long)units * rank / G), u1 = (int)((long long)units * (rank + 1) / G), nrow = 3 * m.nn;
+  // team `team` of the block works on its part v0 + team and every teams-th after it; part v on the units from first(v) on,
+  // in turn over the team's groups
+  const int groups = Shared ? groups_arg : blockDim.x / kBicgUnit, teams = Shared ? blockDim.x / (kBicgUnit * groups) : 1;
+  const int team = Shared ? ug / groups : 0, tg = ug - team * groups;
+  const int v0 = Shared ? V * rank / G : rank, v1 = Shared ? V * (rank + 1) / G : rank + 1, nrow = 3 * m.nn;
+  const int u0 = (int)((long long)units * rank / G), u1 = (int)((long long)units * (rank + 1) / G);  // of the one part
+  auto first = [&](int v) { return Shared ? (int)((long long)units * v / V) : v == rank ? u0 : u1; };
+  auto each_part = [&](auto f) {
+    if constexpr (Shared) {
+      for (int part = v0 + team; part < v1; part += teams) f(part);
+    } else {
+      f(rank);
+    }
+  };
   const size_t np = m.np;
   const double *vals = A.vals, *kinv = A.kinv, *rh = A.rh;
   double *x = A.x, *r = A.r, *p = A.p, *v = A.v, *sv = A.s, *tv = A.t, *y = A.y, *z = A.z;
   BicgState *st = A.st;
   unsigned int *ctr = A.ticket, target = 0;
-  int its = 0, turn = 0, converged = st->converged;
+  int its = 0, turn = 0, buf = 0, converged = st->converged;
   const int max_its = st->max_its;
   const double limit = st->rel_tol * st->r0;
   double rnorm = st->rnorm;
@@ -431,30 +452,36 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDe
     target += G;
     return ok = group_barrier(ctr, target, &s_ok);
   };
-  // s_tot = the sums over all threads of a and b; partials in two buffers in turn, as a block may write the next ones
-  // while another still reads these.
-  auto reduce = [&](double a, double b) {
+  // s_tot = the sums of the a and b that the threads have added up in work(part, a, b) for every part; partials in two
+  // buffers in turn, as a block may write the next ones while another still reads these.
+  auto reduce = [&](auto work) {
+    each_part([&](int part) {
+      double a = 0.0, b = 0.0;
+      work(part, a, b);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, o);
-      b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    if (lane == 0) {
-      s_warp[0][wid] = a;
-      s_warp[1][wid] = b;
-    }
+      for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+      }
+      if (lane == 0) {
+        s_warp[0][part - v0][tg * 9 + (t >> 5)] = a;
+        s_warp[1][part - v0][tg * 9 + (t >> 5)] = b;
+      }
+    });
     __syncthreads();
-    double *part = A.red + (size_t)turn * 2 * G;
+    const int nv = Shared ? V : G;
+    double *parts = A.red + (size_t)turn * 2 * nv;
     turn ^= 1;
-    if (tid < 2) {
+    if (tid < 2 * (v1 - v0)) {
+      const int kind = tid & 1, i = tid >> 1;
       double q = 0.0;
-      for (int w = 0; w < nwarps; ++w) q += s_warp[tid][w];
-      part[(size_t)tid * G + rank] = q;
+      for (int w = 0; w < 9 * groups; ++w) q += s_warp[kind][i][w];
+      parts[(size_t)kind * nv + v0 + i] = q;
     }
     if (!barrier()) return false;
     if (wid < 2) {
       double q = 0.0;
-      for (int b2 = lane; b2 < G; b2 += 32) q += __ldcg(part + (size_t)wid * G + b2);
+      for (int b2 = lane; b2 < nv; b2 += 32) q += __ldcg(parts + (size_t)wid * nv + b2);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) q += __shfl_down_sync(0xffffffffu, q, o);
       if (lane == 0) s_tot[wid] = q;
@@ -462,15 +489,19 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDe
     __syncthreads();
     return true;
   };
-  // f(row) for the rows of this thread
-  auto each_row = [&](auto f) {
-    for (int u = u0 + ug; u < u1; u += groups)
+  // f(row) for the rows of this thread in a part
+  auto part_rows_of = [&](int part, auto f) {
+    const int end = first(part + 1);
+    for (int u = first(part) + tg; u < end; u += groups)
       if (t < 96 && u * 96 + t < nrow) f(u * 96 + t);
   };
-  // f(row, (K in)_row) (K^T in) for the rows of this thread
-  auto product = [&](const double *in, auto f) {
-    int buf = 0;
-    for (int u = u0 + ug; u < u1; u += groups, buf ^= 1) {
+  auto each_row = [&](auto f) {
+    each_part([&](int part) { part_rows_of(part, f); });
+  };
+  // f(row, (K in)_row) (K^T in) for the rows of this thread in a part
+  auto product = [&](int part, const double *in, auto f) {
+    const int end = first(part + 1);
+    for (int u = first(part) + tg; u < end; u += groups, buf ^= 1) {
       const int n = u * 32 + lane;
       int i, j, k;
       double q = 0.0;
@@ -508,12 +539,13 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDe
     }
     if (!barrier()) break;
     // v = K y; alpha = rho / (rh . v)
-    double a = 0.0, b = 0.0;
-    product(y, [&](int row, double q) {
-      v[row] = q;
-      a = fma(rh[row], q, a);
-    });
-    if (!reduce(a, 0.0)) break;
+    if (!reduce([&](int part, double &a, double &) {
+          product(part, y, [&](int row, double q) {
+            v[row] = q;
+            a = fma(rh[row], q, a);
+          });
+        }))
+      break;
     if (tid == 0) {
       s_alpha = s_rho / s_tot[0];
       if (!isfinite(s_alpha) || s_tot[0] == 0.0) s_done = 1;
@@ -530,13 +562,14 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDe
     });
     if (!barrier()) break;
     // t = K z; omega = (t . s) / (t . t)
-    a = b = 0.0;
-    product(z, [&](int row, double q) {
-      tv[row] = q;
-      a = fma(q, sv[row], a);
-      b = fma(q, q, b);
-    });
-    if (!reduce(a, b)) break;
+    if (!reduce([&](int part, double &a, double &b) {
+          product(part, z, [&](int row, double q) {
+            tv[row] = q;
+            a = fma(q, sv[row], a);
+            b = fma(q, q, b);
+          });
+        }))
+      break;
     if (tid == 0) {
       s_omega = s_tot[0] / s_tot[1];
       if (!isfinite(s_omega) || s_tot[1] == 0.0) s_done = 1;
@@ -545,15 +578,16 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1) k_bicg_solve(MeshDe
     if (s_done) break;
     // x += omega z; r = s - omega t; rho, beta and the stop test
     const double omega = s_omega;
-    a = b = 0.0;
-    each_row([&](int row) {
-      x[row] += omega * z[row];
-      const double q = sv[row] - omega * tv[row];
-      r[row] = q;
-      a = fma(rh[row], q, a);
-      b = fma(q, q, b);
-    });
-    if (!reduce(a, b)) break;
+    if (!reduce([&](int part, double &a, double &b) {
+          part_rows_of(part, [&](int row) {
+            x[row] += omega * z[row];
+            const double q = sv[row] - omega * tv[row];
+            r[row] = q;
+            a = fma(rh[row], q, a);
+            b = fma(q, q, b);
+          });
+        }))
+      break;
     its += 1;
     rnorm = sqrt(s_tot[1]);
     converged = rnorm <= limit;
@@ -636,17 +670,22 @@ int mgb_launch_bicg_iter(const MeshDev *m, const AdjDev *A, unsigned int *active
 }
 
 // All iterations after mgb_launch_bicg_init in one cooperative launch; -1 (nothing launched) where that does not pay.
-int mgb_launch_bicg_solve(const MeshDev *m, const AdjDev *A, int transpose, cudaStream_t s) {
+int mgb_launch_bicg_solve(const MeshDev *m, const AdjDev *A, int transpose, int parts, cudaStream_t s) {
   const int sms = coop_sms();
   if (!sms || m->nn > kBicgNodes) return -1;
   int units = (int)cdiv(m->nn, 32);
-  const int per = (int)cdiv(units, sms), groups = per < kBicgGroups ? per : kBicgGroups;
-  const int blocks = (int)cdiv(units, groups) < sms ? (int)cdiv(units, groups) : sms;
+  const int per = (int)cdiv(units, sms);
+  int groups = per < kBicgGroups ? per : kBicgGroups;
+  int V = (int)cdiv(units, groups) < sms ? (int)cdiv(units, groups) : sms;
+  const int share = parts < kBicgShare ? parts : kBicgShare, most = sms > share ? sms / share : 1;
+  const int blocks = V < most ? V : most, teams = (int)cdiv(V, blocks);
+  const int threads = kBicgUnit * groups * (teams < kBicgGroups / groups ? teams : kBicgGroups / groups);
   MeshDev mesh = *m;
   AdjDev adj = *A;
-  void *args[] = {&mesh, &adj, &units};
-  const void *f = transpose ? (const void *)k_bicg_solve<true> : (const void *)k_bicg_solve<false>;
-  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(kBicgUnit * groups), args, 0, s);
+  void *args[] = {&mesh, &adj, &units, &V, &groups};
+  const void *f = blocks < V ? (transpose ? (const void *)k_bicg_solve<true, true> : (const void *)k_bicg_solve<false, true>)
+                             : (transpose ? (const void *)k_bicg_solve<true, false> : (const void *)k_bicg_solve<false, false>);
+  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(threads), args, 0, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
     return -1;

@@ -156,8 +156,9 @@ int mgb_launch_bicg_init(const mgb::MeshDev *m, const mgb::AdjDev *A, cudaStream
 int mgb_launch_bicg_iter(const mgb::MeshDev *m, const mgb::AdjDev *A, unsigned int *active, int transpose,
                          cudaStream_t s);
 // All iterations after mgb_launch_bicg_init in one cooperative launch; -1 (nothing launched) where that does not pay.
-// Where the state's `stalled` is set afterwards nothing was solved, and the ticket is to be cleared.
-int mgb_launch_bicg_solve(const mgb::MeshDev *m, const mgb::AdjDev *A, int transpose, cudaStream_t s);
+// Where the state's `stalled` is set afterwards nothing was solved, and the ticket is to be cleared.  1 / parts of the SMs
+// are taken (a half at least), which changes no result.
+int mgb_launch_bicg_solve(const mgb::MeshDev *m, const mgb::AdjDev *A, int transpose, int parts, cudaStream_t s);
 
 #ifdef __cplusplus
 }

@@ -214,7 +214,7 @@ int Engine::bicg_solve(bool transpose, double *x) {
   launches_ += 1;
   check_launch(mgb_launch_bicg_init(&mesh_, &P.adj, stream_), "bicg init");
   const int chunk = 16;
-  const int one = mgb_launch_bicg_solve(&mesh_, &P.adj, transpose ? 1 : 0, stream_);
+  const int one = mgb_launch_bicg_solve(&mesh_, &P.adj, transpose ? 1 : 0, AtWork::parts(), stream_);
   if (one >= 0) {
     check_launch(one, "bicg solve");
     launches_ += 1;

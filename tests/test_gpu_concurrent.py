@@ -2,6 +2,7 @@
 blocks a solve takes, never its result: every sum has an order that does not depend on them.  (Jacobi solves of many large
 handles in one call are launched kernel by kernel, which rounds the FP64 sums in another order; the sizes here are below.)"""
 import ctypes
+import threading
 import time
 
 import numpy as np
@@ -101,5 +102,45 @@ def test_fast_handles_overlap(gpu_lib):
     import micropp_gb300 as mg
     hs = handles([(25, 1, "damage")] * 13, **dict(wl.FAST_FORM, precond=0, calc_ctan_lin=0), coupling=[mg.FE_FULL])
     assert at_once_over_in_turn(hs) < 0.7
+    for h, _ in hs:
+        h.close()
+
+
+def paths(hs):
+    """A load path and its reverse pass on every handle, each in a thread of its own; results."""
+    out = [None] * len(hs)
+
+    def run(i):
+        h, strains = hs[i]
+        sigma, _ = h.path_forward(np.vstack([0.5 * strains, strains]), PARAMS, 1)
+        gp, gs, _ = h.path_vjp(np.random.default_rng(i).uniform(-1, 1, (2, 6)))
+        out[i] = (sigma, gp, gs, [h.path_newton(k) for k in range(2)])
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(len(hs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    return out
+
+
+PARAMS = np.array([[m[1], m[2], m[5], m[4], m[3]] for m in (MATS["damage"], (0, 1e8, 0.25, 0, 0, 0), MATS["elastic"])])
+
+
+# parts of less than a unit and of one, two and three units at a time, of which a block has one to three
+@pytest.mark.parametrize("sizes", [[3, (7, 4, 9), 16, 12], [20, 17, 21], [23, 26]])
+def test_paths_at_once_are_bitwise_the_lone_ones(gpu_lib, sizes):
+    import micropp_gb300 as mg
+    hs = handles([(n, 1, "damage") for n in sizes], coupling=[mg.FE_FULL], calc_ctan_lin=0, nr_max_its=30, nr_max_tol=1e-30,
+                 nr_rel_tol=1e-11, cg_rel_tol=1e-12, cg_max_its=20000)
+    lone = []
+    for i in range(len(hs)):
+        h, strains = hs[i]
+        sigma, _ = h.path_forward(np.vstack([0.5 * strains, strains]), PARAMS, 1)
+        gp, gs, _ = h.path_vjp(np.random.default_rng(i).uniform(-1, 1, (2, 6)))
+        lone.append((sigma, gp, gs, [h.path_newton(k) for k in range(2)]))
+    for _ in range(2):
+        for a, b in zip(lone, paths(hs)):
+            assert all(np.array_equal(x, y) for x, y in zip(a[:3], b[:3])) and a[3] == b[3]
     for h, _ in hs:
         h.close()
