@@ -19,6 +19,7 @@
 #include <sstream>
 #include <stdexcept>
 
+#include "assembly_ring.h"
 #include "at_work.hpp"
 #include "cuda_util.hpp"
 #include "launch.h"
@@ -241,7 +242,7 @@ Engine::Engine(const micropp3_config &cfg) {
     I.vals = d_A0_;
     upload_insts();
     upload_list({0});
-    launches_ += 2;
+    count_assembly(1, sizeof(double));
     check_launch(mgb_launch_assembly(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, 1, d_ring_, ring_bytes_,
                                      stream_),
                  "A0");
@@ -505,7 +506,7 @@ double Engine::slot_bytes() const {
 // The ring of element matrices that an assembly of n instances works through: two element layers at least, as many as
 // kRingBytes hold beyond that (three quarters of the L2), no more than there are.
 void Engine::ensure_ring(int n, size_t value_bytes) {
-  const size_t layer = (size_t)n * 576 * mesh_.nex * mesh_.ney * value_bytes;
+  const size_t layer = ring_layer_bytes(mesh_.nex, mesh_.ney, n, value_bytes);
   const size_t bytes = std::max(2 * layer, std::min((mesh_.nez + 1) * layer, kRingBytes));
   if (bytes <= ring_bytes_) return;
   clear_graphs();  // captured assemblies hold the old ring
@@ -515,6 +516,11 @@ void Engine::ensure_ring(int n, size_t value_bytes) {
   ring_bytes_ = 0;
   d_ring_ = dalloc<char>(bytes, "element matrices");
   ring_bytes_ = bytes;
+}
+
+// The kernels of an assembly of n instances with the ring as it is, to launches_.
+void Engine::count_assembly(int n, size_t value_bytes) {
+  launches_ += assembly_launches(mesh_.nex, mesh_.ney, mesh_.nez, n, value_bytes, ring_bytes_);
 }
 
 void Engine::ensure_slots(int n) {
@@ -1049,7 +1055,7 @@ void Engine::assemble32(int nlist) {
                  "assembly (FP32 gather)");
   } else {
     timer_begin(t_asm_, (double)nlist * (4.0 * kEllPerNode * mesh_.np + 8.0 * nndim() + 8.0 * nvars()));
-    launches_ += 2;
+    count_assembly(nlist, sizeof(float));
     check_launch(mgb_launch_assembly32(&mesh_, &mats_, d_etype_, d_dsh_, d_ke32_, d_insts_, d_list_, nlist, d_ring_,
                                        ring_bytes_, stream_),
                  "assembly (FP32)");
@@ -1479,7 +1485,7 @@ std::vector<NewtonResult> Engine::newton(const std::vector<int> &slots,
       a0_iteration = true;
     } else {
       timer_begin(t_asm_, (double)na * (8.0 * kEllPerNode * mesh_.np + 8.0 * nndim() + 8.0 * nvars()));
-      launches_ += 2;
+      count_assembly(na, sizeof(double));
       if (exact_tangent_)  // load paths: the exact consistent tangent (quadratic Newton)
         check_launch(mgb_launch_assembly_dual(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, na, d_ring_,
                                               ring_bytes_, stream_),

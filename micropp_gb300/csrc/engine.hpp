@@ -175,6 +175,7 @@ class Engine {
   void residual(const std::vector<int> &slots);
   void cg_solve(const std::vector<int> &slots);
   void ensure_ring(int n, size_t value_bytes);
+  void count_assembly(int n, size_t value_bytes);
   void cg_init(const std::vector<double> &rel_tols, int max_its);
   bool coop32(int n, bool use_mg) const;
   bool coop_solve32(int n, int nr, bool use_mg);

@@ -6,6 +6,7 @@
 // an element, elements around a node); only grid-wide reductions use a tree.
 #include <cuda_runtime.h>
 
+#include "assembly_ring.h"
 #include "device.cuh"
 #include "df.cuh"
 #include "elem_df.cuh"
@@ -793,8 +794,8 @@ static int launch_assembly(const MeshDev *m, const Mats *mats, const int8_t *ety
                            const T *ke_phase, const Inst *insts, const int *list, int nlist, void *ring, size_t bytes,
                            cudaStream_t s) {
   if (nlist <= 0) return 0;
-  const size_t L = (size_t)m->nex * m->ney, fit = bytes / (sizeof(T) * 576 * L * nlist);
-  const int layers = fit < (size_t)m->nez + 1 ? (int)fit : m->nez + 1;
+  const size_t L = (size_t)m->nex * m->ney;
+  const int layers = ring_layers(m->nez, ring_layer_bytes(m->nex, m->ney, nlist, sizeof(T)), bytes);
   if (!ring || layers < 2) return (int)cudaErrorInvalidValue;
   for (int z0 = 0; z0 < m->nez; z0 += layers - 1) {
     const int z1 = z0 + layers - 1 < m->nez ? z0 + layers - 1 : m->nez;

@@ -285,7 +285,7 @@ int Engine::path_vjp(const double *gsigma, double *grad_params, double *grad_str
       I.has_vars_old = 1;
       upload_insts();
       upload_list({0});
-      launches_ += 2;
+      count_assembly(1, sizeof(double));
       check_launch(mgb_launch_assembly_dual(&mesh_, &mats_, d_etype_, d_dsh_, d_ke_, d_insts_, d_list_, 1, d_ring_,
                                             ring_bytes_, stream_),
                    "adjoint tangent");
