@@ -1,6 +1,7 @@
 // assembly_ring.h -- how an assembly by element matrices (fe_kernels.cu) goes through its scratch ring.  Plain host code.
 #pragma once
 
+#include <algorithm>
 #include <cstddef>
 
 namespace mgb {
@@ -8,6 +9,12 @@ namespace mgb {
 // Bytes of the matrices of one element layer of n instances.
 inline size_t ring_layer_bytes(int nex, int ney, int n, size_t value_bytes) {
   return (size_t)n * 576 * nex * ney * value_bytes;
+}
+
+// Bytes of a ring: two element layers at least (a workspace's slots count them), and beyond that as many as `most` (three
+// quarters of the L2) and a tenth of the free memory hold, no more than there are.  More layers mean fewer launches only.
+inline size_t ring_bytes(int nez, size_t layer, size_t most, size_t free_bytes) {
+  return std::max(2 * layer, std::min({((size_t)nez + 1) * layer, most, free_bytes / 10}));
 }
 
 // Element layers that a ring of `bytes` holds, no more than an assembly uses.

@@ -503,19 +503,24 @@ double Engine::slot_bytes() const {
   return b;
 }
 
-// The ring of element matrices that an assembly of n instances works through: two element layers at least, as many as
-// kRingBytes hold beyond that (three quarters of the L2), no more than there are.
+// The ring of element matrices that an assembly of n instances works through.  Slots are taken from 60% of the free memory
+// with two layers each (slot_bytes); the layers beyond come from the rest.
 void Engine::ensure_ring(int n, size_t value_bytes) {
   const size_t layer = ring_layer_bytes(mesh_.nex, mesh_.ney, n, value_bytes);
-  const size_t bytes = std::max(2 * layer, std::min((mesh_.nez + 1) * layer, kRingBytes));
-  if (bytes <= ring_bytes_) return;
-  clear_graphs();  // captured assemblies hold the old ring
-  sync();
-  dfree(d_ring_);
-  d_ring_ = nullptr;
-  ring_bytes_ = 0;
-  d_ring_ = dalloc<char>(bytes, "element matrices");
-  ring_bytes_ = bytes;
+  if (layer <= ring_layer_) return;
+  size_t free_b = 0, total_b = 0;
+  check(cudaMemGetInfo(&free_b, &total_b), "mem info");
+  const size_t bytes = ring_bytes(mesh_.nez, layer, kRingBytes, free_b);
+  if (bytes > ring_bytes_) {
+    clear_graphs();  // captured assemblies hold the old ring
+    sync();
+    dfree(d_ring_);
+    d_ring_ = nullptr;
+    ring_bytes_ = ring_layer_ = 0;
+    d_ring_ = dalloc<char>(bytes, "element matrices");
+    ring_bytes_ = bytes;
+  }
+  ring_layer_ = layer;
 }
 
 // The kernels of an assembly of n instances with the ring as it is, to launches_.

@@ -278,7 +278,7 @@ class Engine {
   int *h_list_ = nullptr;      // pinned: the lists uploaded since the stream was last waited for
   size_t h_list_cap_ = 0, list_used_ = 0;
   char *d_ring_ = nullptr;  // element matrices of a few layers (ensure_ring)
-  size_t ring_bytes_ = 0;
+  size_t ring_bytes_ = 0, ring_layer_ = 0;  // its size, and the largest layer it was sized for
   PathState path_;
   bool graphs_ = true;                         // CG chunks replayed from captured CUDA graphs
   std::map<long, cudaGraphExec_t> graph_cache_;  // (solver, listed instances) -> executable graph
