@@ -138,6 +138,10 @@ void micropp3_set_kernel_timing(struct micropp3 *self, int enable);
 /* CUDA graphs: the CG iterations run in chunks captured once per (solver, batch size) and replayed
  * (default on; chunks are launched directly while kernel timing is on). */
 void micropp3_set_cuda_graphs(struct micropp3 *self, int enable);
+/* Polls after which a block of a one-launch solve gives up waiting for another one; the call then fails with "a linear
+ * solve stalled" and leaves the handle as a failed call does (nothing accepted, usable again).  0: the default, 2^22,
+ * seconds; such a wait ends within microseconds as a rule. */
+void micropp3_set_wait_limit(struct micropp3 *self, unsigned int polls);
 int micropp3_kernel_stats(const struct micropp3 *self, const char *family, long *launches, double *ms,
                           double *bytes);
 

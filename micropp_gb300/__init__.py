@@ -115,6 +115,7 @@ def load():
         "micropp3_path_vjp": (C.c_int, [H, dp, dp, dp]),
         "micropp3_path_newton": (None, [H, C.c_int, ip, ip, ip, dp]),
         "micropp3_set_cuda_graphs": (None, [H, C.c_int]),
+        "micropp3_set_wait_limit": (None, [H, C.c_uint]),
         "micropp3_homogenize_many": (None, [C.POINTER(H), C.c_int]),
         "micropp3_ell_solve_cgpd": (C.c_int, [ip, C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_double,
                                              C.c_int, ip, C.c_void_p]),
@@ -327,6 +328,10 @@ class Micropp:
 
     def set_cuda_graphs(self, on):
         self._call("micropp3_set_cuda_graphs", 1 if on else 0)
+
+    def set_wait_limit(self, polls):
+        """Polls after which a block of a one-launch solve gives up (0: the default); the call then raises."""
+        self._call("micropp3_set_wait_limit", polls)
 
     def path_newton(self, step):
         """(Newton its, CG its, status bits, |b|/|b0|) of a step of the last path."""

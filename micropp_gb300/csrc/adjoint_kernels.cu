@@ -437,6 +437,7 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1)
   unsigned int *ctr = A.ticket, target = 0;
   int its = 0, turn = 0, buf = 0, converged = st->converged;
   const int max_its = st->max_its;
+  const unsigned int polls = st->polls ? st->polls : kSpinLimit;
   const double limit = st->rel_tol * st->r0;
   double rnorm = st->rnorm;
   bool ok = true;
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(kBicgUnit *kBicgGroups, 1)
   const bool skip = s_done != 0;
   auto barrier = [&]() {
     target += G;
-    return ok = group_barrier(ctr, target, &s_ok);
+    return ok = group_barrier(ctr, target, &s_ok, polls);
   };
   // s_tot = the sums of the a and b that the threads have added up in work(part, a, b) for every part; partials in two
   // buffers in turn, as a block may write the next ones while another still reads these.

@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
     double *x = I.du, *r = I.r, *z = I.z, *p = I.p, *Ap = I.Ap;
     const double min_err = cs->min_err, rel_err = cs->rel_err, pnorm0 = cs->pnorm0;
     const int max_its = cs->max_its;
+    const unsigned int polls = I.polls ? I.polls : kSpinLimit;
     if (threadIdx.x == 0) {
       s_rz = cs->rz;
       s_its = 0;
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
     for (int u = u0 + ug; u < u1; u += K)
       if (u * 32 + lane < m.nn) p[fi * np + u * 32 + lane] = z[(u * 32 + lane) * 3 + fi];
     target += G;
-    bool ok = group_barrier(ctr, target, &s_ok);
+    bool ok = group_barrier(ctr, target, &s_ok, polls);
     while (ok) {
       // Ap = A p and p.Ap
       for (int u = u0 + ug, turn = 0; u < u1; u += K, turn ^= 1) {
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
         }
       }
       target += G;
-      if (!(ok = group_barrier(ctr, target, &s_ok))) break;
+      if (!(ok = group_barrier(ctr, target, &s_ok, polls))) break;
       tree_blocks<1>(part, 0, units, sums);
       __syncthreads();
       if (threadIdx.x == 0) s_alpha = s_rz / sum8(sums[0], (units + 7) / 8);
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
         if (lane == 16) upart[uwarps + w] = both;
       }
       target += G;
-      if (!(ok = group_barrier(ctr, target, &s_ok))) break;
+      if (!(ok = group_barrier(ctr, target, &s_ok, polls))) break;
       tree_blocks<2>(upart, uwarps, uwarps, sums);
       __syncthreads();
       if (threadIdx.x == 32) s_beta = sum8(sums[1], ublocks) / s_rz;
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(kUnitThreads *KMAX, 1)
       const double beta = s_beta;
       for (int q = rank * blockDim.x + threadIdx.x; q < 3 * m.np; q += G * blockDim.x) p[q] = fma(beta, p[q], z[q]);
       target += G;
-      if (!(ok = group_barrier(ctr, target, &s_ok))) break;
+      if (!(ok = group_barrier(ctr, target, &s_ok, polls))) break;
     }
     if (threadIdx.x == 0) {
       if (!ok) {  // a block of the group never arrived: reported to the host, which clears the counter

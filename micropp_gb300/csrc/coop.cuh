@@ -27,15 +27,15 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
 }
 
 // Barrier over the G blocks of a group: `ctr` counts arrivals, `target` the count that ends this barrier.  Returns
-// false (in every thread of the block) when the wait ran out.
-__device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int target, int *ok) {
+// false (in every thread of the block) when the wait ran out, after `polls` of them.
+__device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int target, int *ok, unsigned int polls) {
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
     unsigned int spin = 0;
-    while ((int)(ld_acquire(ctr) - target) < 0 && ++spin < kSpinLimit) {
+    while ((int)(ld_acquire(ctr) - target) < 0 && ++spin < polls) {
     }
-    *ok = spin < kSpinLimit;
+    *ok = spin < polls;
   }
   __syncthreads();
   return *ok != 0;

@@ -91,7 +91,7 @@ struct Ctx {
   const float *ks, *vals;
   const double *b;
   double *red;
-  unsigned int *ctr;
+  unsigned int *ctr, polls;
   uint64_t policy;  // L2 eviction priority of the matrix values
   double min_err, rel_err;
   double tot[12], rz[6], pn0[6];
@@ -785,6 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     c.b = I.b;
     c.red = I.red;
     c.ctr = I.ticket;
+    c.polls = I.polls ? I.polls : kSpinLimit;
     c.min_err = NR == 1 ? abs_tol : c6s->min_err;
     c.rel_err = NR == 1 ? rel_tols[a] : c6s->rel_err;
     if (NR == 1) c.rdone[0] = 0;
@@ -796,7 +797,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   bool ok = true;
   auto barrier = [&]() {
     target += G;
-    ok = group_barrier(c.ctr, target, &c.ok);
+    ok = group_barrier(c.ctr, target, &c.ok, c.polls);
     return ok;
   };
   // Sums over the instance of what share(v, w) returns in lane 0 for warp w of the block's part v (the values of warp w

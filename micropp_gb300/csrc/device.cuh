@@ -128,7 +128,7 @@ struct Inst {
   MgInst *mg;              // multigrid hierarchy (NULL: Jacobi-preconditioned CG)
   double strain[6];
   int has_vars_old;        // J2 evolute writes only when a history buffer exists (material.cpp:168-181)
-  int pad;
+  unsigned int polls;      // of a one-launch solve's block at a barrier before it gives up; 0: kSpinLimit
 };
 
 struct Voigt6 {
@@ -139,7 +139,8 @@ struct Voigt6 {
 struct BicgState {
   double rho, rho_old, alpha, omega, beta, r0, rnorm, rel_tol;
   int its, max_its, done, converged;
-  int stalled, pad;     // a one-launch solve waited in vain for one of its blocks
+  int stalled;          // a one-launch solve waited in vain for one of its blocks
+  unsigned int polls;   // as Inst.polls
 };
 
 // Vectors and scratch of the adjoint solve of one RVE (node-interleaved FP64, like u).

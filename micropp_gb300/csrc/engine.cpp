@@ -652,6 +652,7 @@ void Engine::ensure_slots(int n) {
     I.mg = w.mg;
     I.vars_old = nullptr;
     I.vars_new = w.vars_aux;
+    I.polls = polls_;
   }
   if (list_cap_ < n) {
     dfree(d_list_);
@@ -828,6 +829,11 @@ void Engine::clear_graphs() {
   graph_cache_.clear();
   for (auto &kv : newton_graphs_) cudaGraphExecDestroy(kv.second.exec);
   newton_graphs_.clear();
+}
+
+void Engine::set_polls(unsigned int polls) {
+  polls_ = polls;
+  for (Inst &I : h_insts_) I.polls = polls;
 }
 
 void Engine::set_graphs(bool on) {

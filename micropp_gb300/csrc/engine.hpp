@@ -143,6 +143,7 @@ class Engine {
   int mg_levels() const { return mg_ ? (int)mg_mesh_.size() : 0; }
   double last_homogenize_ms() const { return last_ms_; }
   void set_graphs(bool on);
+  void set_polls(unsigned int polls);  // Inst.polls
   bool graphs() const { return graphs_; }
   void set_kernel_timing(bool on);
   bool kernel_stats(const std::string &family, long *launches, double *ms, double *bytes);
@@ -269,6 +270,7 @@ class Engine {
   double last_ms_ = 0.0;
   long total_cg_its_ = 0;
   long long beside_ = 0;
+  unsigned int polls_ = 0;
   long launches_ = 0;  // kernels of this library launched by the handle
   KernelTimer t_spmv_, t_update_, t_asm_, t_res_, t_spmv6_, t_upd6_;
   KernelTimer t_rap_;  // multigrid operators after an assembly: smoother diagonals and Galerkin products

@@ -226,6 +226,10 @@ void micropp3_set_cuda_graphs(struct micropp3 *self, int enable) {
   if (Engine *e = eng(self, "micropp3_set_cuda_graphs")) guard("micropp3_set_cuda_graphs", [&] { e->set_graphs(enable != 0); });
 }
 
+void micropp3_set_wait_limit(struct micropp3 *self, unsigned int polls) {
+  if (Engine *e = eng(self, "micropp3_set_wait_limit")) guard("micropp3_set_wait_limit", [&] { e->set_polls(polls); });
+}
+
 void micropp3_homogenize_many(struct micropp3 *const *handles, int n) {
   if (n <= 0) return;
   if (!handles) {

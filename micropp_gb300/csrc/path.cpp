@@ -208,6 +208,7 @@ int Engine::bicg_solve(bool transpose, double *x) {
   P.adj.red = w.red;
   P.adj.ticket = w.ticket;
   BicgState st{};
+  st.polls = polls_;
   st.rel_tol = std::max(cg_rel_tol_, kAdjTol);
   st.max_its = std::min(std::max(cg_max_its_, 1), kAdjMaxIts);
   check(cudaMemcpyAsync(P.d_st, &st, sizeof(st), cudaMemcpyHostToDevice, stream_), "bicg state");
