@@ -1,8 +1,9 @@
-"""The solves launched kernel by kernel, on batches that the dispatch sends there: the FP64 CG beyond the nodes of one launch and
-Newton iterations as CUDA graphs."""
+"""The solves launched kernel by kernel, on batches that the dispatch sends there: the FP64 CG beyond the nodes of one launch,
+Newton iterations as CUDA graphs, and the fast form's error with the headline's solver."""
 import numpy as np
 import pytest
 
+import test_gpu_fast_error as fast_error
 import test_gpu_one_launch as one_launch
 from cases import gpu_config
 from micropp_gb300 import workloads as wl
@@ -42,3 +43,28 @@ def test_newton_graphs_of_a_launched_batch_match_unfused(gpu_lib):
             assert np.array_equal(a.get_stress(gp), b.get_stress(gp)) and np.array_equal(a.u(gp, 1), b.u(gp, 1))
             assert a.newton(gp) == b.newton(gp) and a.status(gp) == b.status(gp) == mg.STATUS_OK
     assert counts[2] > counts[3], counts
+
+
+@pytest.mark.parametrize("precond", [1, 0], ids=["multigrid", "jacobi"])
+def test_fast_form_error_of_a_launched_batch_at_60cubed(gpu_lib, precond):
+    """Five RVEs of the headline workload in one handle (1.13 million nodes, one launch takes 950,000), two of them against
+    the FP64 solution: the bars of the fast form."""
+    import micropp_gb300 as mg
+    from micropp_gb300 import accuracy
+    n = fast_error.N
+    et, xts, targets = wl.damage_layers_rves(n, 32, 2024)
+    mats = wl.damage_layers_materials(mg, xts[0])
+    fast = accuracy.fast_solution(n, mats, et, 0.5 * targets[:5], targets[:5], dict(wl.FAST_FORM, precond=precond))
+    res = accuracy.compare(fast, fp64_solutions(mats, et, targets))
+    assert all(status == mg.STATUS_OK for _, _, status in fast)
+    assert res["stress"] <= fast_error.TOL_STRESS and res["ctan"] <= fast_error.TOL_CTAN, res
+
+
+FP64 = []
+
+
+def fp64_solutions(mats, et, targets):
+    from micropp_gb300 import accuracy
+    if not FP64:
+        FP64.extend(accuracy.fp64_solution(fast_error.N, mats, et, 0.5 * targets[i], targets[i]) for i in range(2))
+    return FP64
