@@ -102,7 +102,9 @@ void micropp3_clear_error(void);
 
 /* Homogenize several handles at once (RVEs of different sizes, microstructures or materials): each handle's
  * Gauss points form one batch on the handle's own stream, and the handles run concurrently from worker
- * threads.  Do not use the handles from another thread meanwhile. */
+ * threads.  Do not use the handles from another thread meanwhile.  The results are those of micropp3_homogenize on each
+ * handle, bit for bit unless the handles hold more than 250,000 nodes in all: FP32 solves with the Jacobi preconditioner
+ * are then launched kernel by kernel, which adds the FP64 parts of a sum in another order. */
 void micropp3_homogenize_many(struct micropp3 *const *handles, int n);
 
 /* Status word (MICROPP3_STATUS_*) of macro point gp after the last homogenize(). */

@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kNodeBlock) k_bicg_r(MeshDev m, AdjDev A, unsi
 // of the 3 rows and one of the 3 planes of the stencil each, 27 products per thread -- the launched kernels' 243
 // products per thread keep a few SMs busy for tens of microseconds, since an FP64 warp instruction holds its quarter of
 // the SM for 64 cycles.  Rows 96 u .. 96 u + 95 of the vectors belong to the first 96 threads of unit u's group in
-// every phase.  A 12^3 J2 path of 4 steps, forward and reverse: 503 ms launched, 171 ms so.
+// every phase.  A 12^3 J2 path of 4 steps, forward and reverse: 508 ms launched, 138 ms so.
 constexpr int kBicgUnit = 288;  // threads per unit
 constexpr int kBicgGroups = 3;  // units a block works on at a time, at most
 // A sum over the rows is formed over V parts, the blocks of a solve that has all SMs; with half of them (other handles are
@@ -398,7 +398,7 @@ constexpr int kBicgGroups = 3;  // units a block works on at a time, at most
 // each, on all SMs each, on halves, and launched, ms: 4 of 20^3 95.5, 87.5, 90.8, 16 of 16^3 257, 233, 188, 4 of 30^3 274,
 // 261, 262, 8 of 30^3 552, 523, 450; quarters of the SMs are slower again (16 of 20^3 366, halves 345).
 constexpr int kBicgShare = 2, kBicgParts = kBicgShare + 1;
-// Largest RVE (nodes) solved in one launch: the largest it was measured at.  The launched iteration is five kernels and
+// Largest RVE (nodes) solved in one launch: just above the largest it was measured at (91^3 = 753,571).  The launched iteration is five kernels and
 // re-reads the vectors between them; a load step and its reverse pass (damage, edges of 6, 12, 20, 30, 45, 60, 75, 90)
 // take 21.6, 38.6, 61.9, 99, 335, 717, 1792, 2864 ms launched and 9.1, 14.3, 26.6, 74, 230, 568, 1408, 2673 in one
 // launch: the gain shrinks to 7% where the vectors outgrow L2.

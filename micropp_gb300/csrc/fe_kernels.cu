@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(kNodeBlock) k_node_rhs(MeshDev m, const Inst *
 // The ring keeps a layer per instance that the next chunk of layers still needs, and stays in L2 where two layers of all
 // instances do (not 8 x 60^3 in FP64: 265 MB); each chunk is two launches.  Adding the matrices straight into the rows takes 8 launches, one per parity class (else
 // two elements would add into a row at once), which leave small grids with a few blocks each, and scattered
-// read-modify-writes.  us per assembly, so and now: 8 x damage 12^3 1016 and 538, J2 20^3 698 and 512, damage 60^3 7091
-// and 6719 (the FP64 pipe), FP32 J2 50^3 2377 and 1442, exact J2 12^3 745 and 179.
+// read-modify-writes.  us per assembly, so and now: 8 x damage 12^3 1016 and 505, J2 20^3 698 and 511, damage 60^3 7091
+// and 6759 (the FP64 pipe), FP32 J2 50^3 2377 and 1417, exact J2 12^3 745 and 180.
 //
 // Nonlinear laws: the tangents C of the block's 64 Gauss points are formed first, then cxb = (C B) wg is built
 // cooperatively in shared memory and each thread accumulates its row Ke[p][:] += B[:,p]^T cxb -- the reference's

@@ -2,7 +2,7 @@
 // implicit-differentiation ctan.
 //
 // Newton (mixed): the residual b and its norm stay FP64 (fe_kernels.cu); the Jacobian is assembled in FP32
-// (k_elem_mat<float>) and K du = b is solved by Jacobi-preconditioned CG with FP32 vectors and FP64 dot-product
+// (k_elem_ke<float> and k_ke_gather) and K du = b is solved by Jacobi-preconditioned CG with FP32 vectors and FP64 dot-product
 // accumulation.  The FP64 Newton residual is the refinement residual: each Newton step corrects the FP32 solve.
 //
 // ctan (implicit): at the converged state, with K_t the consistent tangent (FP64 Gauss-point tangents, FP32
